@@ -24,7 +24,7 @@ GPU_SO = os.path.join(PKG, "libdg_gpu.so")
 
 HOST_SRC = [os.path.join(CSRC, "dg_host.c")]
 GPU_SRC = [os.path.join(CSRC, f) for f in ("dg_gpu.cu", "dg_noalloc.cu", "dg_k_generic.cu", "dg_k_x2_small.cu",
-                                            "dg_k_x2_mid.cu", "dg_k_x2_large.cu", "dg_k_wave.cu", "dg_k_multi.cu")]
+                                            "dg_k_x2_mid.cu", "dg_k_x2_large.cu", "dg_k_wave.cu", "dg_k_resident.cu", "dg_k_multi.cu")]
 # translation units: (source, extra flags, object tag); dg_k_multi.cu is compiled once per part
 GPU_UNITS = [(src, [], os.path.basename(src)) for src in GPU_SRC if not src.endswith("dg_k_multi.cu")] + \
     [(os.path.join(CSRC, "dg_k_multi.cu"), ["-DDG_MX_PART=%d" % k], "dg_k_multi%d" % k) for k in range(7)]

@@ -1,0 +1,22 @@
+// dg_k_resident.cu — instances of the resident step (k_step_resident): FP32 one shot and two shots
+// per lane, plain and Kahan, and FP64.  Blocks of up to 256 threads keep all their values in
+// registers; the larger ones serve meshes with more lanes per SM.
+#include "dg_kernels.cuh"
+
+namespace dg {
+
+ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan, bool small) {
+  if (kahan) return {k_step_resident<ArithP2<float>, true, 384>, 384};
+  return {k_step_resident<ArithP2<float>, false, 512>, 512};
+}
+ResKernel<ArithP2<float2>> kernel_resident_f2(bool kahan, bool small) {
+  if (kahan) return {k_step_resident<ArithP2<float2>, true, 256>, 256};
+  if (small) return {k_step_resident<ArithP2<float2>, false, 256>, 256};
+  return {k_step_resident<ArithP2<float2>, false, 384>, 384};
+}
+ResKernel<ArithOps<double>> kernel_resident_d(bool small) {
+  if (small) return {k_step_resident<ArithOps<double>, false, 256>, 256};
+  return {k_step_resident<ArithOps<double>, false, 384>, 384};
+}
+
+}  // namespace dg

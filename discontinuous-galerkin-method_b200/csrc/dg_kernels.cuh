@@ -5,6 +5,7 @@
 #pragma once
 #include "dg_common.cuh"
 #include "dg_step_multi.cuh"
+#include "dg_step_resident.cuh"
 #include "dg_step_wave.cuh"
 #include "dg_step_x2.cuh"
 
@@ -22,6 +23,14 @@ using MxFn = void (*)(Ops<float>, Ops2, const MeshDev<float>*, const int2*, Coun
 // the persistent batch k_step_mx_p
 using MxpFn = void (*)(Ops<float>, Ops2, const MeshDev<float>*, MxLoop, Counters*, int);
 
+// the resident step k_step_resident
+template <class A>
+using ResFn = void (*)(typename A::Ops, MeshDev<typename A::R>, Resident, Counters*, long long, int, unsigned);
+template <class A> struct ResKernel {
+  ResFn<A> fn;
+  int max_threads;  // threads per block its registers allow
+};
+
 template <class F> struct HalfPair {
   F v = nullptr;  // velocity half
   F s = nullptr;  // stress half (and the receivers)
@@ -37,6 +46,9 @@ WaveFn kernel_wave(int S, bool kahan, bool persistent);           // dg_k_wave.c
 WaveFn kernel_wave_async(int S, bool kahan);                      // dg_k_wave.cu
 HalfPair<MxFn> kernels_batch(bool kahan);                         // dg_k_multi.cu
 MxpFn kernel_batch_persistent(bool kahan);                        // dg_k_multi.cu
+ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan, bool small);  // dg_k_resident.cu
+ResKernel<ArithP2<float2>> kernel_resident_f2(bool kahan, bool small); // dg_k_resident.cu
+ResKernel<ArithOps<double>> kernel_resident_d(bool small);            // dg_k_resident.cu
 
 // the packed instances, split by shot count over three translation units
 HalfPair<X2Fn> kernels_packed_small(int S, bool kahan, bool pm);  // S = 2..8

@@ -20,6 +20,11 @@ struct Ops2 {
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// (a packed product that feeds a packed sum may come out fused: where both are to round, a branch
+// lies between them, or the product is taken lane by lane, mul2s)
+__device__ __forceinline__ float2 mul2s(float2 a, float2 b) {
+  return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+}
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 // a - b, exactly rounded (b * -1 is exact)
@@ -388,15 +393,14 @@ __device__ __forceinline__ void stress_x2_core(const Ops2& ops, const MeshDev<fl
   for (int i = 0; i < NP; i++) {
     const float2 dxx = fma2(dl2m, X[i], mul2(dlam, Z[i]));
     const float2 dzz = fma2(dlam, X[i], mul2(dl2m, Z[i]));
-    const float2 dxz = mul2(dmu, W[i]);
     if (KAHAN) {
       kahan2(txx[i], cxx[i], dxx);
       kahan2(tzz[i], czz[i], dzz);
-      kahan2(txz[i], cxz[i], dxz);
+      kahan2(txz[i], cxz[i], mul2(dmu, W[i]));
     } else {
       txx[i] = add2(txx[i], dxx);
       tzz[i] = add2(tzz[i], dzz);
-      txz[i] = add2(txz[i], dxz);
+      txz[i] = fma2(dmu, W[i], txz[i]);
     }
     Ue[(12 + i) * PS] = txx[i];
     Ue[(18 + i) * PS] = tzz[i];
@@ -559,7 +563,7 @@ __device__ __forceinline__ void velocity_x2e_body(const Ops2& ops, const MeshDev
   }
   float2 vx[NP], vz[NP], cx[NP], cz[NP];
 #pragma unroll
-  for (int i = 0; i < NP; i++) { vx[i] = mul2(Up[(0 + i) * H], sp[i]); vz[i] = mul2(Up[(6 + i) * H], sp[i]); }
+  for (int i = 0; i < NP; i++) { vx[i] = mul2(Up[(0 + i) * H], sp[i]); vz[i] = mul2s(Up[(6 + i) * H], sp[i]); }
   float2* __restrict__ Cp = nullptr;
   if (KAHAN) {
     Cp = reinterpret_cast<float2*>(m.C) + p;
@@ -683,8 +687,8 @@ __device__ __forceinline__ void stress_x2e_body(const Ops2& ops, const MeshDev<f
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     const float2 a = any_sponge ? __ldg(reinterpret_cast<const float2*>(m.sponge + (long long)i * m.Kp) + p) : f2(1.f);
-    txx[i] = mul2(Up[(12 + i) * H], a);
-    tzz[i] = mul2(Up[(18 + i) * H], a);
+    txx[i] = KAHAN ? mul2(Up[(12 + i) * H], a) : mul2s(Up[(12 + i) * H], a);
+    tzz[i] = KAHAN ? mul2(Up[(18 + i) * H], a) : mul2s(Up[(18 + i) * H], a);
     txz[i] = mul2(Up[(24 + i) * H], a);
     if (KAHAN) {
       cxx[i] = mul2(Cp[(12 + i) * H], a); czz[i] = mul2(Cp[(18 + i) * H], a); cxz[i] = mul2(Cp[(24 + i) * H], a);
@@ -694,15 +698,14 @@ __device__ __forceinline__ void stress_x2e_body(const Ops2& ops, const MeshDev<f
   for (int i = 0; i < NP; i++) {
     const float2 dxx = fma2(dl2m, X[i], mul2(dlam, Z[i]));
     const float2 dzz = fma2(dlam, X[i], mul2(dl2m, Z[i]));
-    const float2 dxz = mul2(dmu, W[i]);
     if (KAHAN) {
       kahan2(txx[i], cxx[i], dxx);
       kahan2(tzz[i], czz[i], dzz);
-      kahan2(txz[i], cxz[i], dxz);
+      kahan2(txz[i], cxz[i], mul2(dmu, W[i]));
     } else {
       txx[i] = add2(txx[i], dxx);
       tzz[i] = add2(tzz[i], dzz);
-      txz[i] = add2(txz[i], dxz);
+      txz[i] = fma2(dmu, W[i], txz[i]);
     }
     Up[(12 + i) * H] = txx[i];
     Up[(18 + i) * H] = tzz[i];
