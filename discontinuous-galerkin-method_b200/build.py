@@ -24,10 +24,13 @@ GPU_SO = os.path.join(PKG, "libdg_gpu.so")
 
 HOST_SRC = [os.path.join(CSRC, "dg_host.c")]
 GPU_SRC = [os.path.join(CSRC, f) for f in ("dg_gpu.cu", "dg_noalloc.cu", "dg_k_generic.cu", "dg_k_x2_small.cu",
-                                            "dg_k_x2_mid.cu", "dg_k_x2_large.cu", "dg_k_wave.cu", "dg_k_resident.cu", "dg_k_multi.cu")]
-# translation units: (source, extra flags, object tag); dg_k_multi.cu is compiled once per part
-GPU_UNITS = [(src, [], os.path.basename(src)) for src in GPU_SRC if not src.endswith("dg_k_multi.cu")] + \
-    [(os.path.join(CSRC, "dg_k_multi.cu"), ["-DDG_MX_PART=%d" % k], "dg_k_multi%d" % k) for k in range(7)]
+                                            "dg_k_x2_mid.cu", "dg_k_x2_large.cu", "dg_k_wave.cu", "dg_k_wave_mid.cu", "dg_k_resident.cu",
+                                            "dg_k_multi.cu")]
+# translation units: (source, extra flags, object tag); dg_k_multi.cu and dg_k_wave_mid.cu are
+# compiled once per part
+_PARTS = {"dg_k_multi.cu": ("DG_MX_PART", 7), "dg_k_wave_mid.cu": ("DG_WAVE_PART", 4)}
+GPU_UNITS = [(src, [], os.path.basename(src)) for src in GPU_SRC if os.path.basename(src) not in _PARTS] + \
+    [(os.path.join(CSRC, f), ["-D%s=%d" % (flag, k)], "%s%d" % (f, k)) for f, (flag, n) in _PARTS.items() for k in range(n)]
 GPU_DEPS = GPU_SRC + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + \
     [os.path.join(INCLUDE, "dg_gpu.h")]
 
@@ -78,7 +81,7 @@ def gpu_library(force: bool = False, log: str | None = None) -> str:
 
         try:
             # the slow units (the batch parts) first
-            order = sorted(range(len(GPU_UNITS)), key=lambda k: not GPU_UNITS[k][2].startswith("dg_k_multi"))
+            order = sorted(range(len(GPU_UNITS)), key=lambda k: not GPU_UNITS[k][1])
             with ThreadPoolExecutor(max_workers=max(1, min(len(GPU_UNITS), os.cpu_count() or 1))) as ex:
                 results = list(ex.map(compile_one, order))
             text = "".join(" ".join(cmd) + "\n" + r.stdout + r.stderr for cmd, r in results)

@@ -50,6 +50,7 @@ template <class V_> struct ArithP2 {  // FP32, the P2 operators of the reference
   using V = V_;
   using R = float;
   struct Ops {};
+  static __device__ __forceinline__ Ops ops(const dg::Ops<float>&) { return {}; }
   static __device__ __forceinline__ V dr(const Ops&, int i, int n, V x, V h) { return v_axpy_c(p2_dr(i * NP + n), x, h); }
   static __device__ __forceinline__ V ds(const Ops&, int i, int n, V x, V h) { return v_axpy_c(p2_ds(i * NP + n), x, h); }
   static __device__ __forceinline__ V lift(const Ops&, int j, int i, int k, V x, V h) {
@@ -61,6 +62,7 @@ template <class R_> struct ArithOps {  // operators from the parameter bank
   using V = R_;
   using R = R_;
   using Ops = dg::Ops<R>;
+  static __device__ __forceinline__ const Ops& ops(const Ops& o) { return o; }
   static __device__ __forceinline__ V dr(const Ops& o, int i, int n, V x, V h) { return v_fma(o.Dr[i * NP + n], x, h); }
   static __device__ __forceinline__ V ds(const Ops& o, int i, int n, V x, V h) { return v_fma(o.Ds[i * NP + n], x, h); }
   static __device__ __forceinline__ V lift(const Ops& o, int j, int i, int k, V x, V h) {

@@ -130,6 +130,13 @@ struct dg_gpu_ctx {
   unsigned* d_mxbar = nullptr;
   int* d_mxerr = nullptr;
   bool x2pm = false; // the two-shot bodies on the plane-major layout (MeshDev::kind 3)
+  // one FP32 mesh on k_velocity / k_stress with the compile-time P2 operators (kind 0, plane-major;
+  // x2 is then the stored shots, for the resident step), and for half steps of a wave_mid context
+  bool gen_p2 = false;
+  bool form_auto = true;  // the step's form is left to the engine (dg_gpu_opts::wavefront = 0)
+  bool wave_ran = false;  // wavefront launches since the error word was last read
+  bool no_halves = false; // no half steps, as for a wavefront context (an automatic one that chose two launches)
+  bool wave_mid = false;  // a wavefront context of a shot count between the powers of two
   bool wave = false;  // one launch per step (k_step_wave / k_step_wave_p), RCM order, schedule in wv
   bool wave_persistent = false;  // k_step_wave_p: resident blocks looping over the tickets
   bool wave_async = false;       // ... with the old values staged in shared memory by cp.async
@@ -166,6 +173,7 @@ struct dg_gpu_ctx {
   int num_sms = 148;
   int block = 256;
   int blocks_v = 0, blocks_t = 0;
+  int half_v = 0, half_t = 0;  // grids of a half step (those two where the step is two launches)
   bool multi = false;
   int graph_steps = 100;
   cudaGraphExec_t graph = nullptr;
@@ -696,14 +704,18 @@ template <class R> void fill_ops(Ops<R>& o, const dg_gpu_mesh& m) {
     }
 }
 
+// threads per element of a mesh's two-launch kernels (but for two elements per thread, kind 1)
+long long lanes_per_element(const dg_gpu_ctx* c, const MeshHostInfo& h) {
+  return h.kind >= 2 || c->gen_p2 ? h.S_pad / 2 : h.S_pad;
+}
+
 // grid and block tables for the current block size
 template <class R> int layout(dg_gpu_ctx* c, std::vector<MeshDev<R>>& md, MeshDev<R>** d_tab) {
   const int B = c->block;
   std::vector<int2> bv, bt;
   for (size_t k = 0; k < md.size(); k++) {
     MeshHostInfo& h = c->mi[k];
-    const long long lanes =
-        h.kind == 1 ? h.Kp / 2 : (h.kind >= 2 ? (long long)h.K * (h.S_pad / 2) : (long long)h.K * h.S_pad);
+    const long long lanes = h.kind == 1 ? h.Kp / 2 : h.K * lanes_per_element(c, h);
     h.elem_blocks = (int)((lanes + B - 1) / B);
     h.rec_blocks = (h.n_rec * h.S_pad + B - 1) / B;
     md[k].n_elem_blocks = h.elem_blocks;
@@ -712,6 +724,8 @@ template <class R> int layout(dg_gpu_ctx* c, std::vector<MeshDev<R>>& md, MeshDe
   }
   c->blocks_v = (int)bv.size();
   c->blocks_t = (int)bt.size();
+  c->half_v = c->blocks_v;
+  c->half_t = c->blocks_t;
   if (c->multi) {
     if (!*d_tab) {
       int rc = c->alloc(d_tab, md.size());
@@ -859,6 +873,23 @@ int build_wave(dg_gpu_ctx* c) {
   return DG_OK;
 }
 
+// the stored shots of the wavefront step for a count between the powers of two (the instances of
+// dg_k_wave_mid.cu and of 32, 64 and 128): the next multiple of 4 up to 40, of 8 above; 0: none
+int wave_shots(int S) {
+  if (S <= 16 || S > 128) return 0;
+  return S <= 40 ? (S + 3) / 4 * 4 : (S + 7) / 8 * 8;
+}
+// Elements x shots from which on the automatic choice is the wavefront step: its fill and drain
+// cost about 16 us a step, and what it saves is HBM traffic, so the two launches are the faster
+// while the state stays in L2 (us a step, two launches / wavefront; FP32: 24,200 x 16 23 / 33,
+// 51,200 x 16 58 / 62, 9,800 x 64 32 / 41, 24,200 x 40 73 / 69, 51,200 x 24 92 / 86, 24,200 x 64 99 / 92;
+// Kahan: 51,200 x 16 86 / 92, 24,200 x 64 144 / 140).  FP32-Kahan without a packed instance spills in
+// the two launches and gives way earlier (9,800 x 24 31 / 30, 9,800 x 40 56 / 46).  DG_WAVE_MIN overrides it.
+long long wave_min(bool kahan, bool packed) {
+  if (const char* e = getenv("DG_WAVE_MIN")) return atoll(e);
+  return kahan && !packed ? 250000 : 1000000;
+}
+
 // shot counts with a two-shot FP32 kernel instance (element-major), and with a plane-major one
 bool x2_supported(int S) { return (S >= 2 && S <= 16 && S % 2 == 0) || S == 32 || S == 64 || S == 128; }
 bool x2pm_supported(int S) { return S >= 2 && S <= 16 && S % 2 == 0; }
@@ -914,7 +945,7 @@ int launch_k(dg_gpu_ctx* c, void (*kernel)(K...), dim3 grid, dim3 block, A&&... 
   } while (0)
 
 int launch_x2(dg_gpu_ctx* c, cudaEvent_t mid, bool hv = true, bool ht = true) {
-  const dim3 bl(c->block), gv(c->blocks_v), gt(c->blocks_t);
+  const dim3 bl(c->block), gv(c->half_v), gt(c->half_t);
   const HalfPair<X2Fn> k = kernels_packed(c->x2, c->kahan, c->x2pm);
   if (!k.v) return fail(DG_ERR_UNSUPPORTED, "no two-shot kernel for this shot count");
   if (hv) DG_LAUNCH(k.v, gv, c->ops2, c->md_f[0], c->d_ctr);
@@ -942,6 +973,7 @@ int launch_wave(dg_gpu_ctx* c) {
   const WaveFn k = as ? kernel_wave_async(c->x2, c->kahan) : kernel_wave(c->x2, c->kahan, c->wave_persistent);
   if (!k) return fail(DG_ERR_UNSUPPORTED, "no wavefront step for this shot count");
   const dim3 bl(c->block), g(c->wave_persistent ? c->blocks_p : c->blocks_v);
+  c->wave_ran = true;
   k<<<g, bl, wave_smem(c), c->stream>>>(c->ops2, c->md_f[0], c->wv, c->d_ctr);
   return DG_OK;
 }
@@ -957,6 +989,16 @@ const void* resident_kernel(const dg_gpu_ctx* c, int* max_threads = nullptr) {
   return c->x2 == 1 ? of(kernel_resident_f1(c->kahan, small)) : of(kernel_resident_f2(c->kahan, small));
 }
 
+// Lanes a block of the resident step can hold, and whether a mesh of K elements of H lanes fits.
+int resident_lanes(const dg_gpu_ctx* c, bool is_double, bool one, bool kahan) {
+  if (is_double) return kernel_resident_d(false).max_threads;
+  return one ? kernel_resident_f1(kahan, false).max_threads : kernel_resident_f2(kahan, false).max_threads;
+}
+bool resident_off() {
+  const char* env = getenv("DG_RESIDENT");
+  return env && atoi(env) == 0;
+}
+
 // The resident step's tables, where a thread for every lane fits on the SMs at once (FP64 and two
 // shots a lane: 56,832 lanes, FP32 one shot 75,776, Kahan 37,888 and 56,832): elements cut into runs
 // of consecutive ones, one block each; every face between two blocks gets a message slot at the
@@ -968,15 +1010,13 @@ const void* resident_kernel(const dg_gpu_ctx* c, int* max_threads = nullptr) {
 // 3,034 x 3 shots FP32 8.1 -> 4.2 (25-step calls), 20,000 FP64 9.7 -> 6.0, FP32 8.2 -> 3.9.
 int build_resident(dg_gpu_ctx* c) {
   const MeshHostInfo& h = c->mi[0];
-  const char* env = getenv("DG_RESIDENT");
-  if (c->multi || c->wave || c->precision == DG_FP64_REF || !(c->is_double || c->x2) || (env && atoi(env) == 0))
+  if (c->multi || (c->wave && !c->form_auto) || c->precision == DG_FP64_REF || !(c->is_double || c->x2) || resident_off())
     return DG_OK;
   const long K = h.K;
   const int H = c->is_double ? h.S_pad : (c->x2 == 1 ? 1 : h.S_pad / 2);
   const size_t vsize = c->is_double || c->x2 > 1 ? 8 : 4;
-  int max_threads = 0, smem_max = 0;
-  c->res_threads = 1024;
-  resident_kernel(c, &max_threads);
+  const int max_threads = resident_lanes(c, c->is_double, c->x2 == 1, c->kahan);
+  int smem_max = 0;
   CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   const long fit = max_threads / H;  // elements a block can hold
   if (c->face_h.empty() || fit < 1 || (K + c->num_sms - 1) / c->num_sms > fit) return DG_OK;
@@ -1123,7 +1163,7 @@ int launch_step(dg_gpu_ctx* c, cudaEvent_t before_t = nullptr, cudaEvent_t mid =
                 int halves = 3) {
   const bool hv = halves & 1, ht = halves & 2;
   const dim3 bl(c->block);
-  const dim3 gv(c->blocks_v), gt(c->blocks_t);
+  const dim3 gv(c->half_v), gt(c->half_t);
   cudaStream_t st = c->stream;
   if (before_t) CK(cudaEventRecord(before_t, st));
   // the two launches of a step of family F (mesh table and block table for a batch)
@@ -1141,6 +1181,9 @@ int launch_step(dg_gpu_ctx* c, cudaEvent_t before_t = nullptr, cudaEvent_t mid =
     const HalfPair<GenFn<double>> k = kernels_fp64(c->multi);
     if (c->multi) DG_TWO(k, c->ops_d, c->md_d[0], c->d_tab_d, c->d_btab_v, c->d_btab_t);
     else DG_TWO(k, c->ops_d, c->md_d[0], (const MeshDev<double>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
+  } else if (c->wave && halves != 3) {  // half steps of a wave_mid context
+    const HalfPair<GenFn<float>> k = kernels_fp32_p2(c->kahan, true);
+    DG_TWO(k, c->ops_f, c->md_f[0], (const MeshDev<float>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
   } else if (c->wave) {  // the whole step in one launch: it is timed as the "velocity" interval
     int rc = launch_wave(c);
     if (rc) return rc;
@@ -1154,11 +1197,11 @@ int launch_step(dg_gpu_ctx* c, cudaEvent_t before_t = nullptr, cudaEvent_t mid =
     if (hv) DG_LAUNCH(k.v, gv, c->ops_f, c->ops2, c->d_tab_f, c->d_btab_v, c->d_ctr);
     if (mid) CK(cudaEventRecord(mid, st));
     if (ht) DG_LAUNCH(k.s, gt, c->ops_f, c->ops2, c->d_tab_f, c->d_btab_t, c->d_ctr);
-  } else if (c->x2) {
+  } else if (c->x2 && !c->gen_p2) {
     int rc = launch_x2(c, mid, hv, ht);
     if (rc) return rc;
   } else {
-    const HalfPair<GenFn<float>> k = kernels_fp32(c->kahan, c->multi);
+    const HalfPair<GenFn<float>> k = c->gen_p2 ? kernels_fp32_p2(c->kahan, true) : kernels_fp32(c->kahan, c->multi);
     if (c->multi) DG_TWO(k, c->ops_f, c->md_f[0], c->d_tab_f, c->d_btab_v, c->d_btab_t);
     else DG_TWO(k, c->ops_f, c->md_f[0], (const MeshDev<float>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
   }
@@ -1233,7 +1276,8 @@ int check_wave(dg_gpu_ctx* c) {
     *c->res_error = 0;
     return fail(DG_ERR_TIMEOUT, "a wait between blocks of the resident step reached its limit");
   }
-  if (!c->wave) return DG_OK;
+  if (!c->wave || (c->resident && !c->wave_ran)) return DG_OK;
+  c->wave_ran = false;
   int err = 0;
   CK(cudaMemcpyAsync(&err, c->wv.error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1277,7 +1321,7 @@ struct TuneChoice {
 
 int apply_choice(dg_gpu_ctx* c, const TuneChoice& t) {
   if (c->wave) {
-    c->wave_persistent = t.persistent != 0;
+    c->wave_persistent = t.persistent != 0 || c->wave_mid;
     c->margin_warps_per_sm = t.margin;
   }
   if (c->mx) c->mx_persistent = t.persistent != 0;
@@ -1318,7 +1362,7 @@ int autotune(dg_gpu_ctx* c, const char* cache) {
       cand.push_back({b, 0, c->margin_warps_per_sm});
       continue;
     }
-    for (int pers = 0; pers < 2; pers++)
+    for (int pers = c->wave_mid ? 1 : 0; pers < 2; pers++)
       for (int mw : {8, 10, 14}) cand.push_back({b, pers, mw});
   }
   const long probe = std::min<long>(8, c->max_steps);
@@ -1436,14 +1480,45 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
                 p.S_pad);
     if (o.variant == 2 && p.kind == 0)
       return fail(DG_ERR_UNSUPPORTED, "no packed FP32 kernel for this mesh (FP32 only; at most 128 shots)");
+    c->form_auto = o.wavefront == 0;
+    // one FP32 mesh of a shot count without packed two-launch kernels: the resident step where it
+    // fits, the wavefront step (padded to the next count it has) where the engine may choose it,
+    // else one (element, shot) per thread; all with the compile-time P2 operators
+    if (!c->multi && !c->is_double && variant == 0 && p.kind == 0) {
+      const int even = meshes[k].n_shots + (meshes[k].n_shots & 1), Sw = wave_shots(meshes[k].n_shots);
+      const long long K = meshes[k].K, lanes = resident_lanes(c.get(), false, false, c->kahan) / (even / 2);
+      size_t free_b = 0, total_b = 0;
+      CK(cudaMemGetInfo(&free_b, &total_b));
+      auto room = [&](int S) { return 30.0 * K * S * 4 * (c->kahan ? 2 : 1) < 0.8 * free_b; };
+      const bool small = lanes * c->num_sms >= K && !resident_off();
+      if (!small && o.wavefront == 0 && Sw && K * meshes[k].n_shots >= wave_min(c->kahan, false) && room(Sw) &&
+          K * (Sw / 2) < (1LL << 31)) {
+        p.kind = 2;
+        p.S_pad = Sw;
+        c->wave_mid = true;
+      } else if (room(even)) {
+        p.S_pad = even;
+        c->gen_p2 = true;
+      }
+    }
     // the wavefront step: one FP32 mesh on the two-shot kernels; automatic = on
     // automatic: from 16 shots on.  Below, a warp covers several elements and the scattered
     // small gathers in RCM order cost more than the HBM traffic the step saves (200k elements:
     // 2 shots 0.096 ms against 0.073 for two launches, 4 shots 0.103 against 0.091, 8 even,
     // 16 shots 0.199 against 0.228; one shot on 2M elements 0.234 against 0.185)
     c->wave = !c->multi && o.wavefront != -1 &&
-              ((p.kind == 2 && wave_supported(p.S_pad) && (p.S_pad >= 16 || o.wavefront == 1)) ||
+              ((p.kind == 2 && (c->wave_mid || wave_supported(p.S_pad)) && (p.S_pad >= 16 || o.wavefront == 1)) ||
                (p.kind == 1 && o.wavefront == 1));
+    // automatic, and the state stays in L2: two launches (a mesh that fits the resident step keeps
+    // the wavefront form, for its other calls)
+    if (c->wave && c->form_auto && !c->wave_mid) {
+      const int fit = resident_off() ? 0 : resident_lanes(c.get(), false, false, c->kahan) / (p.S_pad / 2);
+      if ((long long)fit * c->num_sms < meshes[k].K &&
+          (long long)meshes[k].K * meshes[k].n_shots < wave_min(c->kahan, true)) {
+        c->wave = false;
+        c->no_halves = true;
+      }
+    }
     if (o.wavefront == 1 && !c->wave)
       return fail(DG_ERR_UNSUPPORTED, "the wavefront step needs one FP32 mesh with 1, 2, 4, 8, ..., 128 shots");
     const char* arrays = getenv("DG_REF_ARRAYS");
@@ -1462,7 +1537,7 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
     h.S_pad = p.S_pad;
     h.kind = p.kind;
     if (!c->multi) {
-      c->x2 = p.kind == 1 ? 1 : (p.kind >= 2 ? p.S_pad : 0);
+      c->x2 = p.kind == 1 ? 1 : (p.kind >= 2 || c->gen_p2 ? p.S_pad : 0);
       c->x2pm = p.kind == 3;
     }
     if (c->wave || (n_meshes == 1 && p.K <= 512L * c->num_sms)) {  // wavefront schedule, resident step's tables
@@ -1523,12 +1598,12 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   // slower in it, so that keeps one block per ticket (DG_WAVE_PERSISTENT=0/1 overrides, for tuning)
   c->wave_persistent = c->wave && c->x2 >= 2;
   if (const char* env = getenv("DG_WAVE_PERSISTENT"))
-    if (c->wave) c->wave_persistent = atoi(env) != 0;
+    if (c->wave && !c->wave_mid) c->wave_persistent = atoi(env) != 0;
   // FP32 on the persistent form: the old values staged in shared memory by cp.async (200k x 64
   // batch: 0.6166 against 0.6245 ms a step, the same bits; FP32-Kahan, which stages twice as many,
   // 1.13 against 1.04, keeps the plain form; DG_WAVE_ASYNC=0/1 overrides)
   c->wave_async = c->x2 >= 16 && !c->kahan;
-  if (const char* env = getenv("DG_WAVE_ASYNC")) c->wave_async = c->x2 >= 16 && atoi(env) != 0;
+  if (const char* env = getenv("DG_WAVE_ASYNC")) c->wave_async = c->wave_mid ? !c->kahan : c->x2 >= 16 && atoi(env) != 0;
   if (const char* env = getenv("DG_PDL")) c->pdl = atoi(env) != 0;
   if (c->mx) {
     if ((rc = c->alloc(&c->d_mxbar, 2))) return rc;
@@ -1958,7 +2033,7 @@ int dg_gpu_reset(dg_gpu_ctx* c) {
 
 int dg_gpu_half_step(dg_gpu_ctx* c, int half) {
   if (!c || (half != 0 && half != 1)) return fail(DG_ERR_ARG, "bad arguments");
-  if (c->wave) return fail(DG_ERR_UNSUPPORTED, "half steps need the two-launch step (wavefront = -1)");
+  if ((c->wave && !c->wave_mid) || c->no_halves) return fail(DG_ERR_UNSUPPORTED, "half steps need the two-launch step (wavefront = -1)");
   if (c->part_done) return fail(DG_ERR_STATE, "the other part of the open half step has not run");
   if ((half == 0) == c->half_pending)
     return fail(DG_ERR_STATE, half == 0 ? "velocity half again before the stress half" : "stress half without the velocity half");
@@ -1990,7 +2065,7 @@ static int launch_part(dg_gpu_ctx* c, int half, int part, bool record) {
   const MeshHostInfo& h = c->mi[0];
   const int B = c->block;
   auto blocks = [&](long n) -> int {
-    const long long lanes = h.kind == 1 ? (n + 1) / 2 : (h.kind >= 2 ? n * (long long)(h.S_pad / 2) : n * (long long)h.S_pad);
+    const long long lanes = h.kind == 1 ? (n + 1) / 2 : n * lanes_per_element(c, h);
     return (int)std::min<long long>(h.elem_blocks, (lanes + B - 1) / B);
   };
   const int bB = blocks(c->part_eB), bO = std::max(bB, blocks(c->part_eO));
@@ -1999,13 +2074,13 @@ static int launch_part(dg_gpu_ctx* c, int half, int part, bool record) {
     b0 = h.elem_blocks;
     b1 = h.elem_blocks + 1;
   }
-  const int save_v = c->blocks_v, save_t = c->blocks_t;
-  c->blocks_v = b1 - b0;
-  c->blocks_t = b1 - b0 + (record ? h.rec_blocks : 0);
+  const int save_v = c->half_v, save_t = c->half_t;
+  c->half_v = b1 - b0;
+  c->half_t = b1 - b0 + (record ? h.rec_blocks : 0);
   if (c->is_double) set_window(c->md_d[0], b0, b1); else set_window(c->md_f[0], b0, b1);
   const int rc = launch_step(c, nullptr, nullptr, nullptr, half == 0 ? 1 : 2);
-  c->blocks_v = save_v;
-  c->blocks_t = save_t;
+  c->half_v = save_v;
+  c->half_t = save_t;
   if (c->is_double) set_window(c->md_d[0], 0, h.elem_blocks); else set_window(c->md_f[0], 0, h.elem_blocks);
   return rc;
 }
@@ -2015,7 +2090,7 @@ int dg_gpu_half_step_part(dg_gpu_ctx* c, int half, int part) {
   if (!c || (half != 0 && half != 1) || part < DG_PART_ALL || part > DG_PART_INTERIOR)
     return fail(DG_ERR_ARG, "bad arguments");
   if (part == DG_PART_ALL) return dg_gpu_half_step(c, half);
-  if (c->wave) return fail(DG_ERR_UNSUPPORTED, "half steps need the two-launch step (wavefront = -1)");
+  if ((c->wave && !c->wave_mid) || c->no_halves) return fail(DG_ERR_UNSUPPORTED, "half steps need the two-launch step (wavefront = -1)");
   if (c->multi) return fail(DG_ERR_UNSUPPORTED, "half-step parts need a context of one mesh");
   if (c->halo.empty()) return fail(DG_ERR_STATE, "no halo lists: the parts are defined by the ghosts");
   if (c->part_done) {
@@ -2135,7 +2210,7 @@ int dg_gpu_debug_stall_wave(dg_gpu_ctx* c, int unit) {
     c->mx_spin = unit >= 0 ? (1u << 14) : (1u << 22);
     return DG_OK;
   }
-  if (!c->wave) return fail(DG_ERR_UNSUPPORTED, "this context has no wavefront step");
+  if (!c->wave || c->wave_mid) return fail(DG_ERR_UNSUPPORTED, "this context has no wavefront step");
   if (unit >= c->wv.NU) return fail(DG_ERR_ARG, "unit out of range");
   CK(cudaSetDevice(c->device));
   int* slot = const_cast<int*>(c->wv.wait);
@@ -2201,7 +2276,8 @@ int dg_gpu_stats_get(dg_gpu_ctx* c, dg_gpu_stats* out) {
       c->precision == DG_FP64_REF
           ? 0
           : (c->wave ? (c->wave_persistent ? 6 : 5)
-                     : (c->mx ? (c->mx_persistent ? 8 : 4) : (c->x2 == 1 ? 3 : (c->x2 ? (c->x2pm ? 7 : 2) : 1))));
+                     : (c->mx ? (c->mx_persistent ? 8 : 4)
+                              : (c->gen_p2 ? 1 : (c->x2 == 1 ? 3 : (c->x2 ? (c->x2pm ? 7 : 2) : 1)))));
   c->stats.bytes_per_step = c->wave ? c->bytes_wave : c->bytes_two_pass;
   *out = c->stats;
   return DG_OK;

@@ -7,17 +7,24 @@
 namespace dg {
 
 HalfPair<GenFn<double>> kernels_fp64(bool multi) {
-  if (multi) return {k_velocity<double, false, true>, k_stress<double, false, true>};
-  return {k_velocity<double, false, false>, k_stress<double, false, false>};
+  if (multi) return {k_velocity<ArithOps<double>, false, true>, k_stress<ArithOps<double>, false, true>};
+  return {k_velocity<ArithOps<double>, false, false>, k_stress<ArithOps<double>, false, false>};
 }
 
 HalfPair<GenFn<float>> kernels_fp32(bool kahan, bool multi) {
   if (kahan) {
-    if (multi) return {k_velocity<float, true, true>, k_stress<float, true, true>};
-    return {k_velocity<float, true, false>, k_stress<float, true, false>};
+    if (multi) return {k_velocity<ArithOps<float>, true, true>, k_stress<ArithOps<float>, true, true>};
+    return {k_velocity<ArithOps<float>, true, false>, k_stress<ArithOps<float>, true, false>};
   }
-  if (multi) return {k_velocity<float, false, true>, k_stress<float, false, true>};
-  return {k_velocity<float, false, false>, k_stress<float, false, false>};
+  if (multi) return {k_velocity<ArithOps<float>, false, true>, k_stress<ArithOps<float>, false, true>};
+  return {k_velocity<ArithOps<float>, false, false>, k_stress<ArithOps<float>, false, false>};
+}
+
+HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan, bool two) {
+  if (two && kahan) return {k_velocity<ArithP2<float2>, true, false>, k_stress<ArithP2<float2>, true, false>};
+  if (two) return {k_velocity<ArithP2<float2>, false, false>, k_stress<ArithP2<float2>, false, false>};
+  if (kahan) return {k_velocity<ArithP2<float>, true, false>, k_stress<ArithP2<float>, true, false>};
+  return {k_velocity<ArithP2<float>, false, false>, k_stress<ArithP2<float>, false, false>};
 }
 
 HalfPair<GenFn<double>> kernels_reference(bool multi, bool otf) {

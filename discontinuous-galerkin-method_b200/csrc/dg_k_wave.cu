@@ -4,13 +4,16 @@
 
 namespace dg {
 
+// the resident-block form for the shot counts between the powers of two (dg_k_wave_mid.cu)
+WaveFn kernel_wave_mid(int S, bool kahan);
+
 WaveFn kernel_wave_async(int S, bool kahan) {
 #define DG_WVA(SS, KH) \
   if (S == SS && kahan == KH) return (WaveFn)k_step_wave_p<WaveTwoShotsAsync<SS>, KH>;
   DG_WVA(16, false) DG_WVA(16, true) DG_WVA(32, false) DG_WVA(32, true) DG_WVA(64, false) DG_WVA(64, true)
   DG_WVA(128, false) DG_WVA(128, true)
 #undef DG_WVA
-  return nullptr;
+  return kernel_wave_mid(S, kahan);
 }
 
 WaveFn kernel_wave(int S, bool kahan, bool persistent) {
@@ -22,7 +25,7 @@ WaveFn kernel_wave(int S, bool kahan, bool persistent) {
   DG_WV2(2) DG_WV2(4) DG_WV2(8) DG_WV2(16) DG_WV2(32) DG_WV2(64) DG_WV2(128)
 #undef DG_WV2
 #undef DG_WV
-  return nullptr;
+  return persistent ? kernel_wave_mid(S, kahan) : nullptr;
 }
 
 }  // namespace dg

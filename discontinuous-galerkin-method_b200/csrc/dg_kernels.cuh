@@ -38,11 +38,13 @@ template <class F> struct HalfPair {
 
 HalfPair<GenFn<double>> kernels_fp64(bool multi);                 // dg_k_generic.cu
 HalfPair<GenFn<float>> kernels_fp32(bool kahan, bool multi);      // dg_k_generic.cu
+// one FP32 mesh with the compile-time P2 operators, on any layout; `two`: two shots a thread
+HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan, bool two);     // dg_k_generic.cu
 HalfPair<GenFn<double>> kernels_reference(bool multi, bool otf);  // dg_k_generic.cu
 // S shots (2..128, powers of two), or S = 1 on the one-shot layout
 WaveFn kernel_wave(int S, bool kahan, bool persistent);           // dg_k_wave.cu
 // the resident-block form whose halves stage the element's old values in shared memory
-// (S = 16 .. 128); dynamic shared memory: wave_stage_slots<kahan>() * 32 float2 per warp
+// (S = 16, 20, .. 40, 48, .. 120, 128; FP32-Kahan between the powers of two: the plain form); dynamic shared memory: wave_stage_slots<kahan>() * 32 float2 per warp
 WaveFn kernel_wave_async(int S, bool kahan);                      // dg_k_wave.cu
 HalfPair<MxFn> kernels_batch(bool kahan);                         // dg_k_multi.cu
 MxpFn kernel_batch_persistent(bool kahan);                        // dg_k_multi.cu

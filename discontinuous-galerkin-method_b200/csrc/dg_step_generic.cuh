@@ -1,6 +1,7 @@
 // dg_step_generic.cuh — step kernels in the geometric-factor form for any shot count and for
-// batches of meshes: FP64 and FP32 (plain or Kahan-compensated), one thread per (element, shot),
-// plane-major layout U[plane][e*S + s].
+// batches of meshes: FP64 and FP32 (plain or Kahan-compensated), one thread per lane — an element's
+// shot, or its pair of shots on packed FP32x2 (ArithP2<float2>, even stored shots) — on plane-major
+// state U[plane][e*S + s] (or, for half steps of a wavefront context, element-major).
 //
 // The arithmetic is dg_core.cuh's.  Register budget: one sweep over the faces for both velocity
 // components (each neighbour value gathered once); the stress kernel takes the volume terms first
@@ -13,44 +14,49 @@ namespace dg {
 
 // Velocity half-step: for its own element the sponge on the five fields and the source on Vz
 // (OpenMP_Function.c:25-58), then V += dt L_V(T) (OpenMP_Function.c:75-185), L_V = (1/rho) h.
-template <class R, bool KAHAN>
-__device__ __forceinline__ void velocity_body(const Ops<R>& ops, const MeshDev<R>& m, int lb, long long t) {
-  const int S = m.S;
+template <class A, bool KAHAN, class R = typename A::R>
+__device__ __forceinline__ void velocity_body(const Ops<R>& ops_, const MeshDev<R>& m, int lb, long long t) {
+  using V = typename A::V;
+  constexpr int SV = sizeof(V) / sizeof(R);  // shots of a lane
+  const int H = m.S / SV;                    // lanes of an element
   const long long g = (long long)lb * blockDim.x + threadIdx.x;
-  if (g >= (long long)m.K * S) return;
-  int e, s;
-  if (S == 1) { e = (int)g; s = 0; } else { e = (int)(g / S); s = (int)(g - (long long)e * S); }
-  const long long P = m.P;
-  R* __restrict__ Ug = m.U + g;
+  if (g >= (long long)m.K * H) return;
+  int e, s;  // element, lane
+  if (H == 1) { e = (int)g; s = 0; } else { e = (int)(g / H); s = (int)(g - (long long)e * H); }
+  const typename A::Ops& ops = A::ops(ops_);
+  const long long P = m.PS / SV, ES = m.ES / SV, at = e * ES + s;
+  V* const U = reinterpret_cast<V*>(m.U);
+  V* const C = reinterpret_cast<V*>(m.C);
+  V* __restrict__ Ug = U + at;
 
   const int4 fc = __ldg(m.face + e);
   const auto gm = ld4(m.geo + e);
   const R rx = gm.x, sx = gm.y, rz = gm.z, sz = gm.w;
   const bool own_sponge = fc.w & 1;
   const int codes[3] = {fc.x, fc.y, fc.z};
-  R sp[NP];
+  V sp[NP];
 #pragma unroll
-  for (int i = 0; i < NP; i++) sp[i] = own_sponge ? ldg(m.sponge + (long long)i * m.Kp + e) : R(1);
+  for (int i = 0; i < NP; i++) sp[i] = Bcast<V>::of(own_sponge ? ldg(m.sponge + (long long)i * m.Kp + e) : R(1));
 
-  R txz[NP], hx[NP], hz[NP];
+  V txz[NP], hx[NP], hz[NP];
 #pragma unroll
   for (int i = 0; i < NP; i++) txz[i] = v_mul(Ug[(24 + i) * P], sp[i]);
   {
-    R txx[NP], tzz[NP];
+    V txx[NP], tzz[NP];
 #pragma unroll
     for (int i = 0; i < NP; i++) {
       txx[i] = v_mul(Ug[(12 + i) * P], sp[i]);
       tzz[i] = v_mul(Ug[(18 + i) * P], sp[i]);
     }
-    core_velocity_rhs<ArithOps<R>>(ops, rx, sx, rz, sz, txx, tzz, txz, [&](int j, R (&pxx)[NF], R (&pzz)[NF], R (&pxz)[NF]) {
+    core_velocity_rhs<A>(ops, rx, sx, rz, sz, txx, tzz, txz, [&](int j, V (&pxx)[NF], V (&pzz)[NF], V (&pxz)[NF]) {
       const int code = codes[j];
       if (code < 0) {
 #pragma unroll
-        for (int k = 0; k < NF; k++) { pxx[k] = R(0); pzz[k] = R(0); pxz[k] = R(0); }
+        for (int k = 0; k < NF; k++) { pxx[k] = v_const<V>(0.f); pzz[k] = pxx[k]; pxz[k] = pxx[k]; }
         return;
       }
       const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
-      const R* __restrict__ Un = m.U + ((long long)nb * S + s);
+      const V* __restrict__ Un = U + (nb * ES + s);
 #pragma unroll
       for (int k = 0; k < NF; k++) {
         const int node = face_node(nf, flip ? 2 - k : k);
@@ -61,7 +67,7 @@ __device__ __forceinline__ void velocity_body(const Ops<R>& ops, const MeshDev<R
       if (code & 8) {
 #pragma unroll
         for (int k = 0; k < NF; k++) {
-          const R a = ldg(m.sponge + (long long)face_node(nf, flip ? 2 - k : k) * m.Kp + nb);
+          const V a = Bcast<V>::of(ldg(m.sponge + (long long)face_node(nf, flip ? 2 - k : k) * m.Kp + nb));
           pxx[k] = v_mul(pxx[k], a); pzz[k] = v_mul(pzz[k], a); pxz[k] = v_mul(pxz[k], a);
         }
       }
@@ -69,22 +75,34 @@ __device__ __forceinline__ void velocity_body(const Ops<R>& ops, const MeshDev<R
   }
 
   const R irho = __ldg(&m.mat[e].x);
-  R vx[NP], vz[NP], cvx[NP], cvz[NP];
+  V vx[NP], vz[NP], cvx[NP], cvz[NP];
 #pragma unroll
   for (int i = 0; i < NP; i++) { vx[i] = v_mul(Ug[(0 + i) * P], sp[i]); vz[i] = v_mul(Ug[(6 + i) * P], sp[i]); }
   if (KAHAN) {
 #pragma unroll
-    for (int i = 0; i < NP; i++) { cvx[i] = v_mul(m.C[(0 + i) * P + g], sp[i]); cvz[i] = v_mul(m.C[(6 + i) * P + g], sp[i]); }
+    for (int i = 0; i < NP; i++) { cvx[i] = v_mul(C[(0 + i) * P + at], sp[i]); cvz[i] = v_mul(C[(6 + i) * P + at], sp[i]); }
   }
-  R srcz[NP];
+  V srcz[NP];
 #pragma unroll
-  for (int i = 0; i < NP; i++) srcz[i] = R(0);
-  if (__ldg(m.src_elem + s) == e) {
+  for (int i = 0; i < NP; i++) srcz[i] = v_const<V>(0.f);
+  bool mine[SV], any = false;
+#pragma unroll
+  for (int c = 0; c < SV; c++) {
+    mine[c] = __ldg(m.src_elem + s * SV + c) == e;
+    any = any || mine[c];
+  }
+  if (any) {
     const R w = (R)__ldg(m.wavelet + t);
 #pragma unroll
-    for (int i = 0; i < NP; i++) srcz[i] = v_mul(ldg(m.src_fun + s * NP + i), w);
+    for (int i = 0; i < NP; i++) {
+      R x[SV];
+#pragma unroll
+      for (int c = 0; c < SV; c++) x[c] = mine[c] ? v_mul(ldg(m.src_fun + (s * SV + c) * NP + i), w) : R(0);
+      if constexpr (SV == 2) srcz[i] = make_float2(x[0], x[1]);
+      else srcz[i] = x[0];
+    }
   }
-  const R step = v_mul(m.dt, irho);
+  const V step = Bcast<V>::of(v_mul(m.dt, irho));
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     if (KAHAN) {
@@ -99,11 +117,11 @@ __device__ __forceinline__ void velocity_body(const Ops<R>& ops, const MeshDev<R
   }
   if (KAHAN) {
 #pragma unroll
-    for (int i = 0; i < NP; i++) { m.C[(0 + i) * P + g] = cvx[i]; m.C[(6 + i) * P + g] = cvz[i]; }
+    for (int i = 0; i < NP; i++) { C[(0 + i) * P + at] = cvx[i]; C[(6 + i) * P + at] = cvz[i]; }
   }
 }
 
-template <class R, bool KAHAN, bool MULTI>
+template <class A, bool KAHAN, bool MULTI, class R = typename A::R>
 __global__ void __launch_bounds__(256, 2) k_velocity(const __grid_constant__ Ops<R> ops,
                                                      const __grid_constant__ MeshDev<R> one,
                                                      const MeshDev<R>* __restrict__ tab,
@@ -115,7 +133,7 @@ __global__ void __launch_bounds__(256, 2) k_velocity(const __grid_constant__ Ops
   const long long t = ctr->v;
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->s = t;
   if (t >= m.steps) return;
-  velocity_body<R, KAHAN>(ops, m, lb, t);
+  velocity_body<A, KAHAN>(ops, m, lb, t);
 }
 
 // Stress half-step: T = a T + dt L_T(V) (OpenMP_Function.c:188-306),
@@ -123,17 +141,22 @@ __global__ void __launch_bounds__(256, 2) k_velocity(const __grid_constant__ Ops
 //   Tzz += dt [ l (dxVx + ...) + (l+2m) (dzVz + ...) ]
 //   Txz += dt m [ dxVz + dzVx + sum_j S_j (nz_j dVx + nx_j dVz) ]
 // The trailing blocks of the grid record the receivers (V is final during this kernel).
-template <class R, bool KAHAN>
-__device__ __forceinline__ void stress_body(const Ops<R>& ops, const MeshDev<R>& m, int lb, long long t) {
-  const int S = m.S;
+template <class A, bool KAHAN, class R = typename A::R>
+__device__ __forceinline__ void stress_body(const Ops<R>& ops_, const MeshDev<R>& m, int lb, long long t) {
+  using V = typename A::V;
+  constexpr int SV = sizeof(V) / sizeof(R);  // shots of a lane
+  const int H = m.S / SV;                    // lanes of an element
   const long long g = (long long)lb * blockDim.x + threadIdx.x;
-  if (g >= (long long)m.K * S) return;
-  int e, s;
-  if (S == 1) { e = (int)g; s = 0; } else { e = (int)(g / S); s = (int)(g - (long long)e * S); }
-  const long long P = m.P;
-  R* __restrict__ Ug = m.U + g;
+  if (g >= (long long)m.K * H) return;
+  int e, s;  // element, lane
+  if (H == 1) { e = (int)g; s = 0; } else { e = (int)(g / H); s = (int)(g - (long long)e * H); }
+  const typename A::Ops& ops = A::ops(ops_);
+  const long long P = m.PS / SV, ES = m.ES / SV, at = e * ES + s;
+  V* const U = reinterpret_cast<V*>(m.U);
+  V* const C = reinterpret_cast<V*>(m.C);
+  V* __restrict__ Ug = U + at;
 
-  R vx[NP], vz[NP];
+  V vx[NP], vz[NP];
 #pragma unroll
   for (int i = 0; i < NP; i++) { vx[i] = Ug[(0 + i) * P]; vz[i] = Ug[(6 + i) * P]; }
   const int4 fc = __ldg(m.face + e);
@@ -141,16 +164,16 @@ __device__ __forceinline__ void stress_body(const Ops<R>& ops, const MeshDev<R>&
   const R rx = gm.x, sx = gm.y, rz = gm.z, sz = gm.w;
 
   const int codes[3] = {fc.x, fc.y, fc.z};
-  R X[NP], Z[NP], W[NP];
-  core_strain<ArithOps<R>>(ops, rx, sx, rz, sz, vx, vz, [&](int j, R (&px)[NF], R (&pz)[NF]) {
+  V X[NP], Z[NP], W[NP];
+  core_strain<A>(ops, rx, sx, rz, sz, vx, vz, [&](int j, V (&px)[NF], V (&pz)[NF]) {
     const int code = codes[j];
     if (code < 0) {
 #pragma unroll
-      for (int k = 0; k < NF; k++) { px[k] = R(0); pz[k] = R(0); }
+      for (int k = 0; k < NF; k++) { px[k] = v_const<V>(0.f); pz[k] = px[k]; }
       return;
     }
     const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
-    const R* __restrict__ Un = m.U + ((long long)nb * S + s);
+    const V* __restrict__ Un = U + (nb * ES + s);
 #pragma unroll
     for (int k = 0; k < NF; k++) {
       const int node = face_node(nf, flip ? 2 - k : k);
@@ -161,7 +184,7 @@ __device__ __forceinline__ void stress_body(const Ops<R>& ops, const MeshDev<R>&
 
   const auto mt = ld4(m.mat + e);
   const R lam = mt.y, mu = mt.z, l2m = mt.w;
-  R txx[NP], tzz[NP], txz[NP], cxx[NP], czz[NP], cxz[NP];
+  V txx[NP], tzz[NP], txz[NP], cxx[NP], czz[NP], cxz[NP];
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     txx[i] = Ug[(12 + i) * P];
@@ -171,22 +194,22 @@ __device__ __forceinline__ void stress_body(const Ops<R>& ops, const MeshDev<R>&
   if (KAHAN) {
 #pragma unroll
     for (int i = 0; i < NP; i++) {
-      cxx[i] = m.C[(12 + i) * P + g]; czz[i] = m.C[(18 + i) * P + g]; cxz[i] = m.C[(24 + i) * P + g];
+      cxx[i] = C[(12 + i) * P + at]; czz[i] = C[(18 + i) * P + at]; cxz[i] = C[(24 + i) * P + at];
     }
   }
   if (fc.w & 1) {
 #pragma unroll
     for (int i = 0; i < NP; i++) {
-      const R a = ldg(m.sponge + (long long)i * m.Kp + e);
+      const V a = Bcast<V>::of(ldg(m.sponge + (long long)i * m.Kp + e));
       txx[i] = v_mul(txx[i], a); tzz[i] = v_mul(tzz[i], a); txz[i] = v_mul(txz[i], a);
       if (KAHAN) { cxx[i] = v_mul(cxx[i], a); czz[i] = v_mul(czz[i], a); cxz[i] = v_mul(cxz[i], a); }
     }
   }
-  const R dl2m = v_mul(m.dt, l2m), dlam = v_mul(m.dt, lam), dmu = v_mul(m.dt, mu);
+  const V dl2m = Bcast<V>::of(v_mul(m.dt, l2m)), dlam = Bcast<V>::of(v_mul(m.dt, lam)), dmu = Bcast<V>::of(v_mul(m.dt, mu));
 #pragma unroll
   for (int i = 0; i < NP; i++) {
-    const R dxx = v_fma(dl2m, X[i], v_mul(dlam, Z[i]));
-    const R dzz = v_fma(dlam, X[i], v_mul(dl2m, Z[i]));
+    const V dxx = v_fma(dl2m, X[i], v_mul(dlam, Z[i]));
+    const V dzz = v_fma(dlam, X[i], v_mul(dl2m, Z[i]));
     if (KAHAN) {
       v_kahan(txx[i], cxx[i], dxx);
       v_kahan(tzz[i], czz[i], dzz);
@@ -203,12 +226,12 @@ __device__ __forceinline__ void stress_body(const Ops<R>& ops, const MeshDev<R>&
   if (KAHAN) {
 #pragma unroll
     for (int i = 0; i < NP; i++) {
-      m.C[(12 + i) * P + g] = cxx[i]; m.C[(18 + i) * P + g] = czz[i]; m.C[(24 + i) * P + g] = cxz[i];
+      C[(12 + i) * P + at] = cxx[i]; C[(18 + i) * P + at] = czz[i]; C[(24 + i) * P + at] = cxz[i];
     }
   }
 }
 
-template <class R, bool KAHAN, bool MULTI>
+template <class A, bool KAHAN, bool MULTI, class R = typename A::R>
 __global__ void __launch_bounds__(256, 2) k_stress(const __grid_constant__ Ops<R> ops,
                                                    const __grid_constant__ MeshDev<R> one,
                                                    const MeshDev<R>* __restrict__ tab,
@@ -221,7 +244,7 @@ __global__ void __launch_bounds__(256, 2) k_stress(const __grid_constant__ Ops<R
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->v = t + 1;
   if (t >= m.steps) return;
   if (lb >= m.n_elem_blocks) { record(m, lb - m.n_elem_blocks, t); return; }
-  stress_body<R, KAHAN>(ops, m, lb, t);
+  stress_body<A, KAHAN>(ops, m, lb, t);
 }
 
 }  // namespace dg

@@ -45,7 +45,7 @@ __device__ __forceinline__ void mx_velocity_block(const Ops<float>& ops, const O
         break;
     }
   } else {
-    velocity_body<float, KAHAN>(ops, m, lb, t);
+    velocity_body<ArithOps<float>, KAHAN>(ops, m, lb, t);
   }
 }
 
@@ -83,7 +83,7 @@ __device__ __forceinline__ void mx_stress_block(const Ops<float>& ops, const Ops
         break;
     }
   } else {
-    stress_body<float, KAHAN>(ops, m, lb, t);
+    stress_body<ArithOps<float>, KAHAN>(ops, m, lb, t);
   }
 }
 
