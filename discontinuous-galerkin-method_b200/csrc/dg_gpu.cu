@@ -985,12 +985,14 @@ const void* resident_kernel(const dg_gpu_ctx* c, int* max_threads = nullptr) {
     return (const void*)k.fn;
   };
   const bool small = c->res_threads <= 256;
+  if (c->precision == DG_FP64_REF) return of(kernel_resident_ref());
   if (c->is_double) return of(kernel_resident_d(small));
   return c->x2 == 1 ? of(kernel_resident_f1(c->kahan, small)) : of(kernel_resident_f2(c->kahan, small));
 }
 
 // Lanes a block of the resident step can hold, and whether a mesh of K elements of H lanes fits.
 int resident_lanes(const dg_gpu_ctx* c, bool is_double, bool one, bool kahan) {
+  if (c->precision == DG_FP64_REF) return kernel_resident_ref().max_threads;
   if (is_double) return kernel_resident_d(false).max_threads;
   return one ? kernel_resident_f1(kahan, false).max_threads : kernel_resident_f2(kahan, false).max_threads;
 }
@@ -1000,17 +1002,19 @@ bool resident_off() {
 }
 
 // The resident step's tables, where a thread for every lane fits on the SMs at once (FP64 and two
-// shots a lane: 56,832 lanes, FP32 one shot 75,776, Kahan 37,888 and 56,832): elements cut into runs
+// shots a lane: 56,832 lanes, FP32 one shot 75,776, Kahan and the reference operators 37,888, Kahan one
+// shot 56,832): elements cut into runs
 // of consecutive ones, one block each; every face between two blocks gets a message slot at the
 // element that receives it (numbered in element order, so a block's messages lie together).  A
 // mesh whose face codes are not mutual, or that does not fit, keeps the two-launch step.
 // Blocks of 128 lanes, one warp per scheduler, as long as there are SMs for them: 64 lanes run
 // 1-5 % slower on 500-3,000 elements (more messages), 256 up to 25 % (warps share schedulers).
 // Against two launches a step, same bits (us a step): 512 elements FP64 11.7 -> 4.3 (20-step calls),
-// 3,034 x 3 shots FP32 8.1 -> 4.2 (25-step calls), 20,000 FP64 9.7 -> 6.0, FP32 8.2 -> 3.9.
+// 3,034 x 3 shots FP32 8.1 -> 4.2 (25-step calls), 20,000 FP64 9.7 -> 6.0, FP32 8.2 -> 3.9, reference
+// operators 12.5 -> 8.2.
 int build_resident(dg_gpu_ctx* c) {
   const MeshHostInfo& h = c->mi[0];
-  if (c->multi || (c->wave && !c->form_auto) || c->precision == DG_FP64_REF || !(c->is_double || c->x2) || resident_off())
+  if (c->multi || (c->wave && !c->form_auto) || c->ref_otf || !(c->is_double || c->x2) || resident_off())
     return DG_OK;
   const long K = h.K;
   const int H = c->is_double ? h.S_pad : (c->x2 == 1 ? 1 : h.S_pad / 2);
@@ -1591,8 +1595,7 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(Counters), c->stream));
 
   // automatic block size: 64 threads (measured 2-4 % ahead of 128 and 256 on every family of
-  // the time step: small blocks of these latency-bound kernels end and refill SMs sooner), 256
-  // for the reference-operator kernels
+  // the time step: small blocks of these latency-bound kernels end and refill SMs sooner)
   // persistent wavefront form on the two-shot layout (200k x 64 batch: FP32 605.5 against 578.5 G
   // DOF-updates/s, FP32-Kahan 370.3 against 364.7, the same bits); the one-shot layout runs
   // slower in it, so that keeps one block per ticket (DG_WAVE_PERSISTENT=0/1 overrides, for tuning)
@@ -1614,7 +1617,7 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   // automatic block size: 64 threads for one mesh (see above), 128 for a batch of meshes (its
   // persistent form: 365.5 G DOF-updates/s on the 48-mesh uneven batch against 359.7 at 64
   // threads and 362.8 for two launches a step at 64)
-  int block = o.block_threads ? o.block_threads : (o.precision == DG_FP64_REF ? 256 : (c->mx ? 128 : 64));
+  int block = o.block_threads ? o.block_threads : (c->mx ? 128 : 64);
   if ((rc = set_block(c.get(), block))) return rc;
   // a batch runs persistent when each resident block takes at least 16 work blocks per half, so
   // the two grid barriers of a step cost little against it (DG_MX_PERSISTENT=0/1 overrides)

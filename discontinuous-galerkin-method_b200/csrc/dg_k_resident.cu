@@ -1,5 +1,6 @@
 // dg_k_resident.cu — instances of the resident step (k_step_resident): FP32 one shot and two shots
-// per lane, plain and Kahan, and FP64.  Blocks of up to 256 threads keep all their values in
+// per lane, plain and Kahan, FP64 and the reference
+// operators.  Blocks of up to 256 threads keep all their values in
 // registers; the larger ones serve meshes with more lanes per SM.
 #include "dg_kernels.cuh"
 
@@ -18,5 +19,6 @@ ResKernel<ArithOps<double>> kernel_resident_d(bool small) {
   if (small) return {k_step_resident<ArithOps<double>, false, 256>, 256};
   return {k_step_resident<ArithOps<double>, false, 384>, 384};
 }
+ResKernel<ArithRef> kernel_resident_ref() { return {k_step_resident<ArithRef, false, 256>, 256}; }
 
 }  // namespace dg

@@ -51,6 +51,7 @@ MxpFn kernel_batch_persistent(bool kahan);                        // dg_k_multi.
 ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan, bool small);  // dg_k_resident.cu
 ResKernel<ArithP2<float2>> kernel_resident_f2(bool kahan, bool small); // dg_k_resident.cu
 ResKernel<ArithOps<double>> kernel_resident_d(bool small);            // dg_k_resident.cu
+ResKernel<ArithRef> kernel_resident_ref();                         // dg_k_resident.cu
 
 // the packed instances, split by shot count over three translation units
 HalfPair<X2Fn> kernels_packed_small(int S, bool kahan, bool pm);  // S = 2..8

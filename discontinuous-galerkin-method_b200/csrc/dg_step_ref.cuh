@@ -1,6 +1,7 @@
 // dg_step_ref.cuh — bit-exact reference-operator step kernels (DG_FP64_REF).
 #pragma once
 #include "dg_common.cuh"
+#include "dg_core.cuh"
 
 namespace dg {
 
@@ -49,8 +50,116 @@ __device__ __forceinline__ void ref_rows(const Ops<double>& ops, const MeshDev<d
   }
 }
 
+// The two halves' sums in the reference's order, volume first, then the faces one by one: the
+// accumulator takes the operations the reference gives its sums, ((ab + q[0]) + q[1]) + q[2], and no
+// face's terms are kept.  The loads bound these kernels (72 to 112 operator doubles an element and
+// half), so they run with all the registers one block of 256 threads leaves (254: the compiler asks
+// for many loads at once; 172 registers run 13 % slower) in blocks of 64 (us a step: 57,800 elements
+// 22.6 -> 20.5, 125,000 with Dx, Dz rebuilt 60.1 -> 55.5, 20,000 x 5 shots 31.9 -> 28.0).
+template <bool OTF>
+__device__ __forceinline__ void ref_velocity_volume(const Ops<double>& ops, const MeshDev<double>& m, int e,
+                                                    const double (&txx)[NP], const double (&tzz)[NP],
+                                                    const double (&txz)[NP], double (&ax)[NP], double (&az)[NP]) {
+  const int Kp = m.Kp;
+  const double A0 = __ldg(m.AB + 0 * Kp + e), A1 = __ldg(m.AB + 1 * Kp + e);
+  const double B0 = __ldg(m.AB + 5 * Kp + e), B1 = __ldg(m.AB + 6 * Kp + e);
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    double s1 = 0, s2 = 0, s3 = 0, s4 = 0;
+    double dxr[NP], dzr[NP];
+    ref_rows<OTF>(ops, m, e, i, dxr, dzr);
+#pragma unroll
+    for (int n = 0; n < NP; n++) {
+      s1 = add(s1, mul(dxr[n], txx[n]));
+      s2 = add(s2, mul(dxr[n], txz[n]));
+      s3 = add(s3, mul(dzr[n], tzz[n]));
+      s4 = add(s4, mul(dzr[n], txz[n]));
+    }
+    ax[i] = add(mul(A0, s1), mul(B0, s4));
+    az[i] = add(mul(A1, s2), mul(B1, s3));
+  }
+}
+__device__ __forceinline__ void ref_velocity_face(const Ops<double>& ops, const MeshDev<double>& m, int e, int j,
+                                                  const double (&txx)[NP], const double (&tzz)[NP],
+                                                  const double (&txz)[NP], const double (&pxx)[NF],
+                                                  const double (&pzz)[NF], const double (&pxz)[NF], double (&ax)[NP],
+                                                  double (&az)[NP]) {
+  const long long Kp = m.Kp;
+  double jxx[NF], jzz[NF], jxz[NF];
+#pragma unroll
+  for (int k = 0; k < NF; k++) {
+    const int own = face_node(j, k);
+    jxx[k] = sub(pxx[k], txx[own]); jzz[k] = sub(pzz[k], tzz[own]); jxz[k] = sub(pxz[k], txz[own]);
+  }
+  const double q0 = __ldg(m.Q + (j * 10 + 0) * Kp + e), q1 = __ldg(m.Q + (j * 10 + 1) * Kp + e);
+  const double q2 = __ldg(m.Q + (j * 10 + 2) * Kp + e), q3 = __ldg(m.Q + (j * 10 + 3) * Kp + e);
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    double lxx = 0, lzz = 0, lxz = 0;
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      const double l = ops.L[(j * NP + i) * NF + k];
+      lxx = add(lxx, mul(l, jxx[k])); lzz = add(lzz, mul(l, jzz[k])); lxz = add(lxz, mul(l, jxz[k]));
+    }
+    ax[i] = add(ax[i], add(mul(q0, lxx), mul(q1, lxz)));
+    az[i] = add(az[i], add(mul(q2, lzz), mul(q3, lxz)));
+  }
+}
+template <bool OTF>
+__device__ __forceinline__ void ref_stress_volume(const Ops<double>& ops, const MeshDev<double>& m, int e,
+                                                  const double (&vx)[NP], const double (&vz)[NP], double (&axx)[NP],
+                                                  double (&azz)[NP], double (&axz)[NP]) {
+  const int Kp = m.Kp;
+  double A[5], B[5];
+#pragma unroll
+  for (int q = 2; q < 5; q++) { A[q] = __ldg(m.AB + q * Kp + e); B[q] = __ldg(m.AB + (5 + q) * Kp + e); }
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    double s1 = 0, s2 = 0, s3 = 0, s4 = 0;
+    double dxr[NP], dzr[NP];
+    ref_rows<OTF>(ops, m, e, i, dxr, dzr);
+#pragma unroll
+    for (int n = 0; n < NP; n++) {
+      s1 = add(s1, mul(dxr[n], vx[n]));
+      s2 = add(s2, mul(dxr[n], vz[n]));
+      s3 = add(s3, mul(dzr[n], vx[n]));
+      s4 = add(s4, mul(dzr[n], vz[n]));
+    }
+    axx[i] = add(mul(A[2], s1), mul(B[2], s4));
+    azz[i] = add(mul(A[3], s1), mul(B[3], s4));
+    axz[i] = add(mul(A[4], s2), mul(B[4], s3));
+  }
+}
+__device__ __forceinline__ void ref_stress_face(const Ops<double>& ops, const MeshDev<double>& m, int e, int j,
+                                                const double (&vx)[NP], const double (&vz)[NP], const double (&px)[NF],
+                                                const double (&pz)[NF], double (&axx)[NP], double (&azz)[NP],
+                                                double (&axz)[NP]) {
+  const long long Kp = m.Kp;
+  double jx[NF], jz[NF];
+#pragma unroll
+  for (int k = 0; k < NF; k++) {
+    const int own = face_node(j, k);
+    jx[k] = sub(px[k], vx[own]); jz[k] = sub(pz[k], vz[own]);
+  }
+  double q[6];
+#pragma unroll
+  for (int c = 0; c < 6; c++) q[c] = __ldg(m.Q + (j * 10 + 4 + c) * Kp + e);
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    double lx = 0, lz = 0;
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      const double l = ops.L[(j * NP + i) * NF + k];
+      lx = add(lx, mul(l, jx[k])); lz = add(lz, mul(l, jz[k]));
+    }
+    axx[i] = add(axx[i], add(mul(q[0], lx), mul(q[1], lz)));
+    azz[i] = add(azz[i], add(mul(q[2], lx), mul(q[3], lz)));
+    axz[i] = add(axz[i], add(mul(q[4], lx), mul(q[5], lz)));
+  }
+}
+
 template <bool MULTI, bool OTF>
-__global__ void __launch_bounds__(256) k_velocity_ref(const __grid_constant__ Ops<double> ops,
+__global__ void __launch_bounds__(256, 1) k_velocity_ref(const __grid_constant__ Ops<double> ops,
                                                       const __grid_constant__ MeshDev<double> one,
                                                       const MeshDev<double>* __restrict__ tab,
                                                       const int2* __restrict__ btab,
@@ -89,27 +198,8 @@ __global__ void __launch_bounds__(256) k_velocity_ref(const __grid_constant__ Op
 #pragma unroll
     for (int i = 0; i < NP; i++) vz[i] = add(vz[i], mul(__ldg(m.src_fun + s * NP + i), w));
   }
-  const double A0 = __ldg(m.AB + 0 * Kp + e), A1 = __ldg(m.AB + 1 * Kp + e);
-  const double B0 = __ldg(m.AB + 5 * Kp + e), B1 = __ldg(m.AB + 6 * Kp + e);
-  double abx[NP], abz[NP];
-#pragma unroll
-  for (int i = 0; i < NP; i++) {
-    double s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-    double dxr[NP], dzr[NP];
-    ref_rows<OTF>(ops, m, e, i, dxr, dzr);
-#pragma unroll
-    for (int n = 0; n < NP; n++) {
-      const double dx = dxr[n];
-      const double dz = dzr[n];
-      s1 = add(s1, mul(dx, txx[n]));
-      s2 = add(s2, mul(dx, txz[n]));
-      s3 = add(s3, mul(dz, tzz[n]));
-      s4 = add(s4, mul(dz, txz[n]));
-    }
-    abx[i] = add(mul(A0, s1), mul(B0, s4));
-    abz[i] = add(mul(A1, s2), mul(B1, s3));
-  }
-  double qx[NF][NP], qz[NF][NP];
+  double ax[NP], az[NP];
+  ref_velocity_volume<OTF>(ops, m, e, txx, tzz, txz, ax, az);
   const int codes[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
@@ -131,36 +221,18 @@ __global__ void __launch_bounds__(256) k_velocity_ref(const __grid_constant__ Op
         }
       }
     }
-    double jxx[NF], jzz[NF], jxz[NF];
-#pragma unroll
-    for (int k = 0; k < NF; k++) {
-      const int own = face_node(j, k);
-      jxx[k] = sub(pxx[k], txx[own]); jzz[k] = sub(pzz[k], tzz[own]); jxz[k] = sub(pxz[k], txz[own]);
-    }
-    const double q0 = __ldg(m.Q + (j * 10 + 0) * (long long)Kp + e), q1 = __ldg(m.Q + (j * 10 + 1) * (long long)Kp + e);
-    const double q2 = __ldg(m.Q + (j * 10 + 2) * (long long)Kp + e), q3 = __ldg(m.Q + (j * 10 + 3) * (long long)Kp + e);
-#pragma unroll
-    for (int i = 0; i < NP; i++) {
-      double lxx = 0, lzz = 0, lxz = 0;
-#pragma unroll
-      for (int k = 0; k < NF; k++) {
-        const double l = ops.L[(j * NP + i) * NF + k];
-        lxx = add(lxx, mul(l, jxx[k])); lzz = add(lzz, mul(l, jzz[k])); lxz = add(lxz, mul(l, jxz[k]));
-      }
-      qx[j][i] = add(mul(q0, lxx), mul(q1, lxz));
-      qz[j][i] = add(mul(q2, lzz), mul(q3, lxz));
-    }
+    ref_velocity_face(ops, m, e, j, txx, tzz, txz, pxx, pzz, pxz, ax, az);
   }
   const double dt = m.dt;
 #pragma unroll
   for (int i = 0; i < NP; i++) {
-    Ug[(0 + i) * P] = add(mul(add(add(add(abx[i], qx[0][i]), qx[1][i]), qx[2][i]), dt), vx[i]);
-    Ug[(6 + i) * P] = add(mul(add(add(add(abz[i], qz[0][i]), qz[1][i]), qz[2][i]), dt), vz[i]);
+    Ug[(0 + i) * P] = add(mul(ax[i], dt), vx[i]);
+    Ug[(6 + i) * P] = add(mul(az[i], dt), vz[i]);
   }
 }
 
 template <bool MULTI, bool OTF>
-__global__ void __launch_bounds__(256) k_stress_ref(const __grid_constant__ Ops<double> ops,
+__global__ void __launch_bounds__(256, 1) k_stress_ref(const __grid_constant__ Ops<double> ops,
                                                     const __grid_constant__ MeshDev<double> one,
                                                     const MeshDev<double>* __restrict__ tab,
                                                     const int2* __restrict__ btab,
@@ -194,29 +266,8 @@ __global__ void __launch_bounds__(256) k_stress_ref(const __grid_constant__ Ops<
       txx[i] = mul(txx[i], a); tzz[i] = mul(tzz[i], a); txz[i] = mul(txz[i], a);
     }
   }
-  double A[5], B[5];
-#pragma unroll
-  for (int q = 0; q < 5; q++) { A[q] = __ldg(m.AB + q * Kp + e); B[q] = __ldg(m.AB + (5 + q) * Kp + e); }
-  double abxx[NP], abzz[NP], abxz[NP];
-#pragma unroll
-  for (int i = 0; i < NP; i++) {
-    double s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-    double dxr[NP], dzr[NP];
-    ref_rows<OTF>(ops, m, e, i, dxr, dzr);
-#pragma unroll
-    for (int n = 0; n < NP; n++) {
-      const double dx = dxr[n];
-      const double dz = dzr[n];
-      s1 = add(s1, mul(dx, vx[n]));
-      s2 = add(s2, mul(dx, vz[n]));
-      s3 = add(s3, mul(dz, vx[n]));
-      s4 = add(s4, mul(dz, vz[n]));
-    }
-    abxx[i] = add(mul(A[2], s1), mul(B[2], s4));
-    abzz[i] = add(mul(A[3], s1), mul(B[3], s4));
-    abxz[i] = add(mul(A[4], s2), mul(B[4], s3));
-  }
-  double fxx[NF][NP], fzz[NF][NP], fxz[NF][NP];
+  double axx[NP], azz[NP], axz[NP];
+  ref_stress_volume<OTF>(ops, m, e, vx, vz, axx, azz, axz);
   const int codes[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
@@ -234,34 +285,14 @@ __global__ void __launch_bounds__(256) k_stress_ref(const __grid_constant__ Ops<
         px[k] = Un[(0 + node) * P]; pz[k] = Un[(6 + node) * P];
       }
     }
-    double jx[NF], jz[NF];
-#pragma unroll
-    for (int k = 0; k < NF; k++) {
-      const int own = face_node(j, k);
-      jx[k] = sub(px[k], vx[own]); jz[k] = sub(pz[k], vz[own]);
-    }
-    double q[6];
-#pragma unroll
-    for (int c = 0; c < 6; c++) q[c] = __ldg(m.Q + (j * 10 + 4 + c) * (long long)Kp + e);
-#pragma unroll
-    for (int i = 0; i < NP; i++) {
-      double lx = 0, lz = 0;
-#pragma unroll
-      for (int k = 0; k < NF; k++) {
-        const double l = ops.L[(j * NP + i) * NF + k];
-        lx = add(lx, mul(l, jx[k])); lz = add(lz, mul(l, jz[k]));
-      }
-      fxx[j][i] = add(mul(q[0], lx), mul(q[1], lz));
-      fzz[j][i] = add(mul(q[2], lx), mul(q[3], lz));
-      fxz[j][i] = add(mul(q[4], lx), mul(q[5], lz));
-    }
+    ref_stress_face(ops, m, e, j, vx, vz, px, pz, axx, azz, axz);
   }
   const double dt = m.dt;
 #pragma unroll
   for (int i = 0; i < NP; i++) {
-    Ug[(12 + i) * P] = add(mul(add(add(add(abxx[i], fxx[0][i]), fxx[1][i]), fxx[2][i]), dt), txx[i]);
-    Ug[(18 + i) * P] = add(mul(add(add(add(abzz[i], fzz[0][i]), fzz[1][i]), fzz[2][i]), dt), tzz[i]);
-    Ug[(24 + i) * P] = add(mul(add(add(add(abxz[i], fxz[0][i]), fxz[1][i]), fxz[2][i]), dt), txz[i]);
+    Ug[(12 + i) * P] = add(mul(axx[i], dt), txx[i]);
+    Ug[(18 + i) * P] = add(mul(azz[i], dt), tzz[i]);
+    Ug[(24 + i) * P] = add(mul(axz[i], dt), txz[i]);
   }
 }
 

@@ -24,6 +24,7 @@
 #pragma once
 #include "dg_common.cuh"
 #include "dg_core.cuh"
+#include "dg_step_ref.cuh"
 
 namespace dg {
 
@@ -147,6 +148,15 @@ __device__ __forceinline__ V* state_at(R* U, const MeshDev<R>& m, int e, int pla
   return reinterpret_cast<V*>(U + (long long)e * m.ES + plane * m.PS) + q;
 }
 
+// The reference's own operators and operation order (DG_FP64_REF), for k_step_resident.
+struct ArithRef {
+  using V = double;
+  using R = double;
+  using Ops = dg::Ops<double>;
+};
+template <class A> constexpr bool is_ref = false;
+template <> constexpr bool is_ref<ArithRef> = true;
+
 // `nsteps` steps from step t0.  The stresses held between two steps carry the sponge factor of
 // the coming step already (those in global memory do not), so neighbours read them as they are;
 // the stress tag of step s is seq + s, the velocity tag seq + s + 1.
@@ -159,6 +169,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
   using V = typename A::V;
   using R = typename A::R;
   constexpr int SV = sizeof(V) / sizeof(R);  // shots of a lane
+  constexpr bool REF = is_ref<A>;
   extern __shared__ __align__(16) unsigned char res_smem[];
   V* const sV = reinterpret_cast<V*>(res_smem);  // [12][nls] Vx, Vz
   V* const sT = sV + 12 * w.nls;                 // [18][nls] Txx, Tzz, Txz, sponge factor applied
@@ -224,6 +235,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
     // ---- velocity half: sponge, source, V += dt L_V(T) ----
     {
       V hx[NP], hz[NP];
+      if constexpr (REF)
+        if (mine) ref_velocity_volume<false>(ops, m, e, txx, tzz, txz, hx, hz);
       for (int u = u0; u < NG; u += blockDim.x) {
         V v[9];
         recv_msgs(w.pt + s0 + u, w.ps, tag_t, w, dead, v);
@@ -235,8 +248,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
       }
       __syncthreads();
       if (mine) {
+        if constexpr (!REF) {
 #pragma unroll
-        for (int i = 0; i < NP; i++) { hx[i] = v_const<V>(0.f); hz[i] = hx[i]; }
+          for (int i = 0; i < NP; i++) { hx[i] = v_const<V>(0.f); hz[i] = hx[i]; }
+        }
 #pragma unroll
         for (int j = 0; j < NF; j++) {
           V pxx[NF], pzz[NF], pxz[NF];
@@ -247,9 +262,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
             pzz[k] = p[6 * nls];
             pxz[k] = p[12 * nls];
           }
-          core_velocity_face<A>(ops, j, rx, sx, rz, sz, txx, tzz, txz, pxx, pzz, pxz, hx, hz);
+          if constexpr (REF) ref_velocity_face(ops, m, e, j, txx, tzz, txz, pxx, pzz, pxz, hx, hz);
+          else core_velocity_face<A>(ops, j, rx, sx, rz, sz, txx, tzz, txz, pxx, pzz, pxz, hx, hz);
         }
-        core_velocity_volume<A>(ops, rx, sx, rz, sz, txx, tzz, txz, hx, hz);
+        if constexpr (!REF) core_velocity_volume<A>(ops, rx, sx, rz, sz, txx, tzz, txz, hx, hz);
         if (sponge) {
 #pragma unroll
           for (int i = 0; i < NP; i++) {
@@ -280,6 +296,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
           if constexpr (KAHAN) {
             v_kahan(vx[i], cc[i], v_mul(st, hx[i]));
             v_kahan(vz[i], cc[6 + i], v_fma(st, hz[i], sv[i]));
+          } else if constexpr (REF) {
+            if (src) vz[i] = v_add(vz[i], sv[i]);
+            vx[i] = v_add(v_mul(hx[i], m.dt), vx[i]);
+            vz[i] = v_add(v_mul(hz[i], m.dt), vz[i]);
           } else {
             vx[i] = v_fma(st, hx[i], vx[i]);
             vz[i] = v_fma(st, hz[i], v_add(vz[i], sv[i]));
@@ -293,7 +313,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
     // ---- stress half: T = a T + dt L_T(V) ----
     {
       V X[NP], Z[NP], W[NP];
-      if (mine) core_strain_volume<A>(ops, rx, sx, rz, sz, vx, vz, X, Z, W);
+      if (mine) {
+        if constexpr (REF) ref_stress_volume<false>(ops, m, e, vx, vz, X, Z, W);
+        else core_strain_volume<A>(ops, rx, sx, rz, sz, vx, vz, X, Z, W);
+      }
       for (int u = u0; u < NG; u += blockDim.x) {
         V v[6];
         recv_msgs(w.pv + s0 + u, w.ps, tag_v, w, dead, v);
@@ -314,7 +337,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
             px[k] = p[0];
             pz[k] = p[6 * nls];
           }
-          core_strain_face<A>(ops, j, rx, sx, rz, sz, vx, vz, px, pz, X, Z, W);
+          if constexpr (REF) ref_stress_face(ops, m, e, j, vx, vz, px, pz, X, Z, W);
+          else core_strain_face<A>(ops, j, rx, sx, rz, sz, vx, vz, px, pz, X, Z, W);
         }
         const V a2 = Bcast<V>::of(dl2m), al = Bcast<V>::of(dlam), am = Bcast<V>::of(dmu);
         const bool last = s == nsteps - 1;
@@ -329,6 +353,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
             v_kahan(txx[i], cc[12 + i], dxx);
             v_kahan(tzz[i], cc[18 + i], dzz);
             v_kahan(txz[i], cc[24 + i], v_mul(am, W[i]));
+          } else if constexpr (REF) {  // X, Z, W are the three stresses' rates
+            txx[i] = v_add(v_mul(X[i], m.dt), txx[i]);
+            tzz[i] = v_add(v_mul(Z[i], m.dt), tzz[i]);
+            txz[i] = v_add(v_mul(W[i], m.dt), txz[i]);
           } else {
             txx[i] = v_add(txx[i], dxx);
             tzz[i] = v_add(tzz[i], dzz);

@@ -39,7 +39,7 @@ def _run(m, shots, precision, chunks, **kw):
 # 101: 20,402, more than 128 elements on every SM; 150: 45,000, FP64 and FP32 blocks of 305
 @pytest.mark.parametrize("cells,shots", [(2, 1), (8, 1), (9, 1), (50, 1), (101, 1), (150, 1), (9, 2), (17, 3), (40, 14),
                                          (61, 5)])
-@pytest.mark.parametrize("precision", ["fp64", "fp32", "fp32_kahan"])
+@pytest.mark.parametrize("precision", ["fp64", "fp64_ref", "fp32", "fp32_kahan"])
 def test_resident_equals_two_launches(precision, cells, shots, monkeypatch):
     m = _mesh(cells, shots, precision)
     monkeypatch.setenv("DG_RESIDENT", "0")
@@ -47,7 +47,7 @@ def test_resident_equals_two_launches(precision, cells, shots, monkeypatch):
     monkeypatch.setenv("DG_RESIDENT", "1")
     one, got = _run(m, shots, precision, (1, 2, STEPS - 3))
     assert two == 2 * STEPS
-    lanes = 2 * cells * cells * (shots if precision == "fp64" else (shots + 1) // 2)
+    lanes = 2 * cells * cells * (shots if precision.startswith("fp64") else (shots + 1) // 2)
     if lanes <= 148 * 256:
         assert one == 3
     for a, b in zip(want, got):
