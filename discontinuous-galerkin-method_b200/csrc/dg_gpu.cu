@@ -204,6 +204,12 @@ struct dg_gpu_ctx {
   StepMark marks[kMarks];
   int mark_next = 0;
   cudaEvent_t ev_fetch = nullptr, ev_wavelet = nullptr;
+  // pinned staging of small wavelet updates (dg_gpu_set_wavelet), used in turn; each half has an
+  // event after its last copy, waited for before the half is used again
+  static constexpr int kWave = 256;  // doubles a half
+  double* wave_host = nullptr;
+  int wave_half = 0, wave_pos = 0;  // where the next update goes
+  cudaEvent_t ev_wave[2] = {nullptr, nullptr};
 
   ~dg_gpu_ctx() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -220,6 +226,9 @@ struct dg_gpu_ctx {
     if (ev_wavelet) cudaEventDestroy(ev_wavelet);
     if (snap_host) cudaFreeHost(snap_host);
     if (res_error) cudaFreeHost(res_error);
+    for (auto& e : ev_wave)
+      if (e) cudaEventDestroy(e);
+    if (wave_host) cudaFreeHost(wave_host);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     for (void* p : allocs) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
@@ -2241,6 +2250,33 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   for (int k = k0; k < k1; k++)
     if (t0 + n > c->mi[k].steps) return fail(DG_ERR_ARG, "wavelet window beyond a mesh's steps");
   CK(cudaSetDevice(c->device));
+  // a few samples (a driver that sends each step's): through the staging buffer on the context
+  // stream, behind the steps enqueued and ahead of the next, without a wait (1.8 us a call against
+  // 8 with the copy stream, its event and the wait)
+  const long few = (long)(k1 - k0) * n;
+  if (few > 0 && few <= 64) {
+    if (!c->wave_host) {
+      void* p = nullptr;
+      if (cudaMallocHost(&p, 2 * dg_gpu_ctx::kWave * sizeof(double)) != cudaSuccess)
+        return fail(DG_ERR_NOMEM, "pinned wavelet staging");
+      c->wave_host = (double*)p;
+      for (auto& e : c->ev_wave) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    if (c->wave_pos + few > dg_gpu_ctx::kWave) {  // the half is full: on to the other
+      CK(cudaEventRecord(c->ev_wave[c->wave_half], c->stream));
+      c->wave_half ^= 1;
+      c->wave_pos = 0;
+      CK(cudaEventSynchronize(c->ev_wave[c->wave_half]));
+    }
+    double* const st = c->wave_host + c->wave_half * dg_gpu_ctx::kWave + c->wave_pos;
+    c->wave_pos += (int)few;
+    memcpy(st, w, few * sizeof(double));
+    for (int k = k0; k < k1; k++) {
+      const double* dw = c->is_double ? c->md_d[k].wavelet : c->md_f[k].wavelet;
+      CK(cudaMemcpyAsync((void*)(dw + t0), st + (size_t)(k - k0) * n, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    }
+    return DG_OK;
+  }
   // samples that no enqueued step reads (t0 at or past the steps enqueued so far) go over the
   // copy stream, and the context stream waits for them, so steps in flight keep running;
   // otherwise the copy follows the enqueued steps on the context stream

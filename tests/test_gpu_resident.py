@@ -83,3 +83,28 @@ def test_a_wait_that_runs_out_reports_timeout_and_the_context_recovers(monkeypat
             assert ei.value.code == -10
         e.reset()
         assert e.steps_done == 0 and not np.any(e.fetch("Vz"))
+
+
+@pytest.mark.parametrize("n", [1, 3, 64, 65])
+def test_wavelet_samples_sent_step_by_step(n):
+    """Small wavelet updates go through a staging buffer without a wait: samples sent ahead of their
+    steps, many times around the buffer and reusing the caller's array at once, give the steps of
+    the whole table."""
+    m = _mesh(8, 1, "fp64")
+    total = 650
+    w = np.random.default_rng(8).standard_normal(total) * 1e-2
+    m["wavelet"] = np.zeros(total)
+    with eng.Engine(m, "fp64") as a, eng.Engine(m, "fp64") as b:
+        a.set_wavelet(0, w)
+        a.step(total)
+        buf = np.empty(n)
+        for t in range(0, total, n):
+            k = min(n, total - t)
+            buf[:k] = w[t:t + k]
+            b.set_wavelet(t, buf[:k])
+            buf[:] = np.nan
+            b.step_async(k)
+        b.synchronize()
+        for f in FIELDS:
+            assert np.array_equal(a.fetch(f), b.fetch(f))
+        assert np.abs(a.fetch("Vz")).max() > 0
