@@ -11,13 +11,13 @@
 //                           at compile-time offsets; a warp of S = 64 shots is one element).
 //   geo     R4[Kp]  rx, sx, rz, sz (inverse Jacobian, as fun_DG.c:1162-1165)
 //   mat     R4[Kp]  1/rho, lambda, mu, lambda + 2 mu (the distinct entries of A/B, fun_DG.c:1076-1086)
-//   face    int4[Kp] three face codes and a flag word (see face_code below)
+//   face    int4[Kp] three neighbours and a word of nodes and flags (see below)
 //   sponge  R[6][Kp] absorb_fun, read only for elements whose flag says they are in the sponge
 //
-// Face code: -1 on the outer boundary (exterior state 0, Edge_flag = 0, fun_DG.c:720-738),
-// else nb << 4 | nb_in_sponge << 3 | nb_face << 1 | flip, where nb is the neighbour element,
-// nb_face its face that touches ours and flip says its face nodes run the other way
-// (NeighborNodes, fun_DG.c:1195-1276).
+// Face word (int4): the three neighbours (internal element, -1 on the outer boundary: exterior state 0,
+// Edge_flag = 0, fun_DG.c:720-738) and in w: bit 0 the element is in the sponge, bits 1..3 neighbour j
+// is, bits 4 + 9j + 3k the neighbour's node that touches this element's face j, position k
+// (NeighborNodes, fun_DG.c:1195-1276), three bits each: a gather's node is one shift and one mask.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -34,6 +34,10 @@ constexpr unsigned long long FACE_NODES = 0x245210035ULL;
 __host__ __device__ __forceinline__ int face_node(int j, int k) {
   return (int)((FACE_NODES >> (4 * (3 * j + k))) & 15ULL);
 }
+
+// of a face word's w: the neighbour's node at face j, position k, and whether neighbour j is in the sponge
+__host__ __device__ __forceinline__ int nb_node(int w, int j, int k) { return ((unsigned)w >> (4 + 9 * j + 3 * k)) & 7; }
+__host__ __device__ __forceinline__ bool nb_sponge(int w, int j) { return ((unsigned)w >> (1 + j)) & 1; }
 
 // The P2 operators on the reference triangle for the node order of the reference's operator
 // files (FeketeNew: (1,-1), (0,0), (-1,1), (0,-1), (-1,0), (-1,-1)).  Every entry is a multiple

@@ -140,7 +140,7 @@ struct dg_gpu_ctx {
   bool wave = false;  // one launch per step (k_step_wave / k_step_wave_p), RCM order, schedule in wv
   bool wave_persistent = false;  // k_step_wave_p: resident blocks looping over the tickets
   bool wave_async = false;       // ... with the old values staged in shared memory by cp.async
-  int margin_warps_per_sm = 10;  // lag margin of the wavefront step beyond the unit bandwidth
+  int margin_warps_per_sm = 12;  // lag margin of the wavefront step beyond the unit bandwidth
   int blocks_p = 0;              // its grid
   Wave wv{};
   int stall_unit = -1, stall_saved = 0;  // wait-list entry replaced by dg_gpu_debug_stall_wave
@@ -274,7 +274,8 @@ struct Prepared {
   std::vector<int> new_of_old;  // caller -> internal
   std::vector<double> geo;      // [Kp][4] rx sx rz sz
   std::vector<double> mat;      // [Kp][4] 1/rho lambda mu lambda+2mu
-  std::vector<int4> face;       // [Kp]
+  std::vector<int4> face;       // [Kp] face codes: -1 outer, else neighbour << 4 | its sponge flag << 3 |
+                                // its face << 1 | flip (its nodes run the other way); w: own sponge flag
   std::vector<double> sponge;   // [6][Kp]
   std::vector<int> src_elem;
   std::vector<double> src_fun;  // [S][6]
@@ -627,8 +628,24 @@ int upload_mesh(dg_gpu_ctx* c, const dg_gpu_mesh& m, Prepared& p, MeshDev<R>& d)
   if ((rc = c->upload(&m4, mat))) return rc;
   d.geo = g4;
   d.mat = m4;
+  // face words (dg_common.cuh) from the host's codes
+  std::vector<int4> words(p.face.size());
+#pragma omp parallel for schedule(static)
+  for (size_t n = 0; n < words.size(); n++) {
+    const int code[3] = {p.face[n].x, p.face[n].y, p.face[n].z};
+    int nb[3];
+    unsigned w = p.face[n].w & 1;
+    for (int j = 0; j < 3; j++) {
+      nb[j] = code[j] < 0 ? -1 : code[j] >> 4;
+      if (code[j] < 0) continue;
+      if (code[j] & 8) w |= 2u << j;
+      for (int k = 0; k < 3; k++)
+        w |= (unsigned)face_node((code[j] >> 1) & 3, code[j] & 1 ? 2 - k : k) << (4 + 9 * j + 3 * k);
+    }
+    words[n] = make_int4(nb[0], nb[1], nb[2], (int)w);
+  }
   int4* f4;
-  if ((rc = c->upload(&f4, p.face))) return rc;
+  if ((rc = c->upload(&f4, words))) return rc;
   d.face = f4;
   R* sp;
   if ((rc = c->upload(&sp, cast<R>(p.sponge)))) return rc;
@@ -2165,9 +2182,9 @@ int dg_gpu_halo_lists(dg_gpu_ctx* c, int mesh, long n_send, const long* send, lo
     for (long n = 0; n < h.K; n++) {
       if (ghost[n]) continue;
       eO = n + 1;
-      const int codes[3] = {face[n].x, face[n].y, face[n].z};
+      const int nbs[3] = {face[n].x, face[n].y, face[n].z};
       for (int f = 0; f < 3; f++)
-        if (codes[f] >= 0 && ghost[codes[f] >> 4]) eB = n + 1;
+        if (nbs[f] >= 0 && ghost[nbs[f]]) eB = n + 1;
     }
     c->part_eB = eB;
     c->part_eO = eO;

@@ -33,7 +33,7 @@ __device__ __forceinline__ void velocity_body(const Ops<R>& ops_, const MeshDev<
   const auto gm = ld4(m.geo + e);
   const R rx = gm.x, sx = gm.y, rz = gm.z, sz = gm.w;
   const bool own_sponge = fc.w & 1;
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
   V sp[NP];
 #pragma unroll
   for (int i = 0; i < NP; i++) sp[i] = Bcast<V>::of(own_sponge ? ldg(m.sponge + (long long)i * m.Kp + e) : R(1));
@@ -49,25 +49,24 @@ __device__ __forceinline__ void velocity_body(const Ops<R>& ops_, const MeshDev<
       tzz[i] = v_mul(Ug[(18 + i) * P], sp[i]);
     }
     core_velocity_rhs<A>(ops, rx, sx, rz, sz, txx, tzz, txz, [&](int j, V (&pxx)[NF], V (&pzz)[NF], V (&pxz)[NF]) {
-      const int code = codes[j];
-      if (code < 0) {
+      const int nb = nbs[j];
+      if (nb < 0) {
 #pragma unroll
         for (int k = 0; k < NF; k++) { pxx[k] = v_const<V>(0.f); pzz[k] = pxx[k]; pxz[k] = pxx[k]; }
         return;
       }
-      const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
       const V* __restrict__ Un = U + (nb * ES + s);
 #pragma unroll
       for (int k = 0; k < NF; k++) {
-        const int node = face_node(nf, flip ? 2 - k : k);
+        const int node = nb_node(fc.w, j, k);
         pxx[k] = Un[(12 + node) * P];
         pzz[k] = Un[(18 + node) * P];
         pxz[k] = Un[(24 + node) * P];
       }
-      if (code & 8) {
+      if (nb_sponge(fc.w, j)) {
 #pragma unroll
         for (int k = 0; k < NF; k++) {
-          const V a = Bcast<V>::of(ldg(m.sponge + (long long)face_node(nf, flip ? 2 - k : k) * m.Kp + nb));
+          const V a = Bcast<V>::of(ldg(m.sponge + (long long)nb_node(fc.w, j, k) * m.Kp + nb));
           pxx[k] = v_mul(pxx[k], a); pzz[k] = v_mul(pzz[k], a); pxz[k] = v_mul(pxz[k], a);
         }
       }
@@ -163,20 +162,19 @@ __device__ __forceinline__ void stress_body(const Ops<R>& ops_, const MeshDev<R>
   const auto gm = ld4(m.geo + e);
   const R rx = gm.x, sx = gm.y, rz = gm.z, sz = gm.w;
 
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
   V X[NP], Z[NP], W[NP];
   core_strain<A>(ops, rx, sx, rz, sz, vx, vz, [&](int j, V (&px)[NF], V (&pz)[NF]) {
-    const int code = codes[j];
-    if (code < 0) {
+    const int nb = nbs[j];
+    if (nb < 0) {
 #pragma unroll
       for (int k = 0; k < NF; k++) { px[k] = v_const<V>(0.f); pz[k] = px[k]; }
       return;
     }
-    const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
     const V* __restrict__ Un = U + (nb * ES + s);
 #pragma unroll
     for (int k = 0; k < NF; k++) {
-      const int node = face_node(nf, flip ? 2 - k : k);
+      const int node = nb_node(fc.w, j, k);
       px[k] = Un[(0 + node) * P];
       pz[k] = Un[(6 + node) * P];
     }

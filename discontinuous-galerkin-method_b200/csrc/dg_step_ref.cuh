@@ -200,22 +200,21 @@ __global__ void __launch_bounds__(256, 1) k_velocity_ref(const __grid_constant__
   }
   double ax[NP], az[NP];
   ref_velocity_volume<OTF>(ops, m, e, txx, tzz, txz, ax, az);
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
-    const int code = codes[j];
+    const int nb = nbs[j];
     double pxx[NF], pzz[NF], pxz[NF];
-    if (code < 0) {
+    if (nb < 0) {
 #pragma unroll
       for (int k = 0; k < NF; k++) { pxx[k] = 0.0; pzz[k] = 0.0; pxz[k] = 0.0; }
     } else {
-      const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
       const double* Un = m.U + ((long long)nb * S + s);
 #pragma unroll
       for (int k = 0; k < NF; k++) {
-        const int node = face_node(nf, flip ? 2 - k : k);
+        const int node = nb_node(fc.w, j, k);
         pxx[k] = Un[(12 + node) * P]; pzz[k] = Un[(18 + node) * P]; pxz[k] = Un[(24 + node) * P];
-        if (code & 8) {
+        if (nb_sponge(fc.w, j)) {
           const double a = __ldg(m.sponge + (long long)node * Kp + nb);
           pxx[k] = mul(pxx[k], a); pzz[k] = mul(pzz[k], a); pxz[k] = mul(pxz[k], a);
         }
@@ -268,20 +267,19 @@ __global__ void __launch_bounds__(256, 1) k_stress_ref(const __grid_constant__ O
   }
   double axx[NP], azz[NP], axz[NP];
   ref_stress_volume<OTF>(ops, m, e, vx, vz, axx, azz, axz);
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
-    const int code = codes[j];
+    const int nb = nbs[j];
     double px[NF], pz[NF];
-    if (code < 0) {
+    if (nb < 0) {
 #pragma unroll
       for (int k = 0; k < NF; k++) { px[k] = 0.0; pz[k] = 0.0; }
     } else {
-      const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
       const double* Un = m.U + ((long long)nb * S + s);
 #pragma unroll
       for (int k = 0; k < NF; k++) {
-        const int node = face_node(nf, flip ? 2 - k : k);
+        const int node = nb_node(fc.w, j, k);
         px[k] = Un[(0 + node) * P]; pz[k] = Un[(6 + node) * P];
       }
     }

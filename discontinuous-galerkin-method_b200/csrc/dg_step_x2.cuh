@@ -99,33 +99,32 @@ __device__ __forceinline__ void velocity_x2_body(const Ops2& ops, const MeshDev<
   for (int i = 0; i < NP; i++) { hx[i] = f2(0.f); hz[i] = f2(0.f); }
 
   // surface terms: sum_j S_j (nx_j dTxx + nz_j dTxz), sum_j S_j (nz_j dTzz + nx_j dTxz)
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
-    const int code = codes[j];
+    const int nb = nbs[j];
     float nxs, nzs;
     if (j == 0) { nxs = -0.5f * gm.y; nzs = -0.5f * gm.w; }
     else if (j == 1) { nxs = 0.5f * (gm.x + gm.y); nzs = 0.5f * (gm.z + gm.w); }
     else { nxs = -0.5f * gm.x; nzs = -0.5f * gm.z; }
     const float2 nx = f2(nxs), nz = f2(nzs);
     float2 pxx[NF], pzz[NF], pxz[NF];
-    if (code < 0) {
+    if (nb < 0) {
 #pragma unroll
       for (int k = 0; k < NF; k++) { pxx[k] = f2(0.f); pzz[k] = f2(0.f); pxz[k] = f2(0.f); }
     } else {
-      const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
       const float2* __restrict__ Un = reinterpret_cast<const float2*>(m.U) + (long long)nb * EO + q;
 #pragma unroll
       for (int k = 0; k < NF; k++) {
-        const int node = face_node(nf, flip ? 2 - k : k);
+        const int node = nb_node(fc.w, j, k);
         pxx[k] = Un[(12 + node) * PS];
         pzz[k] = Un[(18 + node) * PS];
         pxz[k] = Un[(24 + node) * PS];
       }
-      if (code & 8) {
+      if (nb_sponge(fc.w, j)) {
 #pragma unroll
         for (int k = 0; k < NF; k++) {
-          const int node = face_node(nf, flip ? 2 - k : k);
+          const int node = nb_node(fc.w, j, k);
           const float2 a = f2(__ldg(m.sponge + (long long)node * m.Kp + nb));
           pxx[k] = mul2(pxx[k], a); pzz[k] = mul2(pzz[k], a); pxz[k] = mul2(pxz[k], a);
         }
@@ -251,7 +250,7 @@ __device__ __forceinline__ float2 ld_v(const float2* p) {
   return *p;
 }
 
-// The per-element constants of the stress update: face codes, geometric factors, materials.
+// The per-element constants of the stress update: face words, geometric factors, materials.
 struct StressConst {
   int4 fc;
   float4 gm, mt;
@@ -307,25 +306,24 @@ __device__ __forceinline__ void stress_x2_core(const Ops2& ops, const MeshDev<fl
     W[i] = fma2(rx, drz, fma2(sx, dsz, fma2(rz, drx, mul2(sz, dsx))));
   }
 
-  const int codes[3] = {fc.x, fc.y, fc.z};
+  const int nbs[3] = {fc.x, fc.y, fc.z};
 #pragma unroll
   for (int j = 0; j < NF; j++) {
-    const int code = codes[j];
+    const int nb = nbs[j];
     float nxs, nzs;
     if (j == 0) { nxs = -0.5f * gm.y; nzs = -0.5f * gm.w; }
     else if (j == 1) { nxs = 0.5f * (gm.x + gm.y); nzs = 0.5f * (gm.z + gm.w); }
     else { nxs = -0.5f * gm.x; nzs = -0.5f * gm.z; }
     const float2 nx = f2(nxs), nz = f2(nzs);
     float2 px[NF], pz[NF];
-    if (code < 0) {
+    if (nb < 0) {
 #pragma unroll
       for (int k = 0; k < NF; k++) { px[k] = f2(0.f); pz[k] = f2(0.f); }
     } else {
-      const int nb = code >> 4, nf = (code >> 1) & 3, flip = code & 1;
       const float2* __restrict__ Un = reinterpret_cast<const float2*>(m.U) + (long long)nb * EO + q;
 #pragma unroll
       for (int k = 0; k < NF; k++) {
-        const int node = face_node(nf, flip ? 2 - k : k);
+        const int node = nb_node(fc.w, j, k);
         px[k] = ld_v<FRESH>(Un + (0 + node) * PS);
         pz[k] = ld_v<FRESH>(Un + (6 + node) * PS);
       }
@@ -444,24 +442,23 @@ __global__ void __launch_bounds__(256, 2) k_stress_x2(const __grid_constant__ Op
 
 __device__ __forceinline__ int pick(const int4& f, int j) { return j == 0 ? f.x : (j == 1 ? f.y : f.z); }
 
-// Decode one lane's face code into a load address that is always valid (element 0 across an
-// outer face), the neighbour's three face nodes in our order, a 0/1 mask and the sponge flag,
-// so all gathers of a face can be issued without branches.
+// One lane's face j: a load address that is always valid (element 0 across an outer face), the
+// neighbour's three face nodes in our order, a 0/1 mask and the sponge flag, so all gathers of a
+// face can be issued without branches.
 struct FaceLane {
   int nb;
   int node[NF];
   float mask;
   bool sponge;
 };
-__device__ __forceinline__ FaceLane face_lane(int code) {
+__device__ __forceinline__ FaceLane face_lane(const int4& w, int j) {
   FaceLane f;
-  const bool v = code >= 0;
-  f.nb = v ? (code >> 4) : 0;
-  const int nf = v ? ((code >> 1) & 3) : 0, fl = v ? (code & 1) : 0;
+  const int nb = pick(w, j);
+  f.nb = max(nb, 0);
 #pragma unroll
-  for (int k = 0; k < NF; k++) f.node[k] = face_node(nf, fl ? 2 - k : k);
-  f.mask = v ? 1.f : 0.f;
-  f.sponge = v && (code & 8);
+  for (int k = 0; k < NF; k++) f.node[k] = nb_node(w.w, j, k);
+  f.mask = nb >= 0 ? 1.f : 0.f;
+  f.sponge = nb_sponge(w.w, j);
   return f;
 }
 // FRESH: values other blocks of the same launch wrote (the wavefront step), read through L2
@@ -508,7 +505,7 @@ __device__ __forceinline__ void velocity_x2e_body(const Ops2& ops, const MeshDev
     if (j == 0) { nx = mul2(f2(-0.5f), sx); nz = mul2(f2(-0.5f), sz); }
     else if (j == 1) { nx = mul2(f2(0.5f), add2(rx, sx)); nz = mul2(f2(0.5f), add2(rz, sz)); }
     else { nx = mul2(f2(-0.5f), rx); nz = mul2(f2(-0.5f), rz); }
-    const FaceLane a = face_lane(pick(f0, j)), b = face_lane(pick(f1, j));
+    const FaceLane a = face_lane(f0, j), b = face_lane(f1, j);
     float2 pxx[NF], pzz[NF], pxz[NF];
 #pragma unroll
     for (int k = 0; k < NF; k++) {
@@ -650,7 +647,7 @@ __device__ __forceinline__ void stress_x2e_body(const Ops2& ops, const MeshDev<f
     else if (j == 1) { nx = mul2(f2(0.5f), add2(rx, sx)); nz = mul2(f2(0.5f), add2(rz, sz)); }
     else { nx = mul2(f2(-0.5f), rx); nz = mul2(f2(-0.5f), rz); }
     // the velocity fields carry no sponge factor in this pass: raw neighbour values
-    const FaceLane a = face_lane(pick(f0, j)), b = face_lane(pick(f1, j));
+    const FaceLane a = face_lane(f0, j), b = face_lane(f1, j);
     float2 px[NF], pz[NF];
 #pragma unroll
     for (int k = 0; k < NF; k++) {
