@@ -96,6 +96,7 @@ template <class R> struct MeshDev {
   int kind;               // FP32 kernel body: 0 one (element, shot) per thread, plane-major;
                           // 1 two elements per thread (S = 1); 2 two shots per thread, element-major
   int sponge_elems;
+  int back;               // the stress half takes the element blocks backwards (stress_block)
   R dt;
   R* U;                   // [30][P]
   R* C;                   // Kahan compensation [30][P] (FP32_KAHAN) or null
@@ -176,6 +177,14 @@ __device__ __forceinline__ const MeshDev<R>* pick_mesh(const MeshDev<R>& one, co
   return tab + b.x;
 }
 
+
+// The stress half's element block for launch block `local`.  Backwards (MeshDev::back, states that
+// do not fit L2): the element blocks in descending order, so that the half starts where the
+// velocity half ended and finds those values in L2, where a sweep in one direction finds none.
+// Then the recorder blocks.
+template <class R> __device__ __forceinline__ int stress_block(const MeshDev<R>& m, int local) {
+  return m.back && local < m.n_elem_blocks ? m.n_elem_blocks - 1 - (local - m.block0) : local;
+}
 
 // Receiver gather of the reference's Record (OpenMP_Function.c:61-72, stride 2): thread q of
 // the recorder blocks copies V at (receiver element, node) for one (receiver, shot).

@@ -730,6 +730,22 @@ template <class R> void fill_ops(Ops<R>& o, const dg_gpu_mesh& m) {
     }
 }
 
+// Whether the state and the elements' constants of all meshes leave L2 (126 MB) between one sweep and
+// the next.  There the two halves sweep in opposite directions (us a step, 133 MB: 388,000 elements
+// FP64 69.9 -> 62.9; 81 MB: 80,000 x 8 42.4 -> 40.2; 105 MB: 627,000 FP32 60.5 -> 52.9; 563 MB: 2 M Kahan
+// 279 -> 270; 12 uneven meshes, 620 MB 400 -> 392), and the wavefront step alternates (200,000 x 64
+// 688 -> 675, 102,000 x 16 Kahan 168 -> 160, 49,400 x 24 82 -> 76); it costs
+// 1-4 % where everything stays in L2 (66 MB: 205,000 FP64 28.3 -> 29.1).  DG_BACK=0/1 overrides it.
+bool larger_than_l2(const dg_gpu_ctx* c) {
+  if (const char* e = getenv("DG_BACK")) return atoi(e) != 0;
+  double bytes = 0;
+  for (const MeshHostInfo& h : c->mi) {
+    const double w = c->is_double ? 8 : 4;
+    bytes += h.K * (30.0 * h.S_pad * w * (c->kahan ? 2 : 1) + 8 * w + 16);
+  }
+  return bytes > 75e6;
+}
+
 // threads per element of a mesh's two-launch kernels (but for two elements per thread, kind 1)
 long long lanes_per_element(const dg_gpu_ctx* c, const MeshHostInfo& h) {
   return h.kind >= 2 || c->gen_p2 ? h.S_pad / 2 : h.S_pad;
@@ -746,8 +762,14 @@ template <class R> int layout(dg_gpu_ctx* c, std::vector<MeshDev<R>>& md, MeshDe
     h.rec_blocks = (h.n_rec * h.S_pad + B - 1) / B;
     md[k].n_elem_blocks = h.elem_blocks;
     for (int b = 0; b < h.elem_blocks; b++) bv.push_back(make_int2((int)k, b));
-    for (int b = 0; b < h.elem_blocks + h.rec_blocks; b++) bt.push_back(make_int2((int)k, b));
   }
+  // past L2 the stress half takes the element blocks backwards (stress_block); then the recorder blocks
+  const bool back = larger_than_l2(c);
+  for (auto& m : md) m.back = back;
+  bt = bv;
+  if (back) std::reverse(bt.begin(), bt.end());
+  for (size_t k = 0; k < md.size(); k++)
+    for (int b = 0; b < c->mi[k].rec_blocks; b++) bt.push_back(make_int2((int)k, c->mi[k].elem_blocks + b));
   c->blocks_v = (int)bv.size();
   c->blocks_t = (int)bt.size();
   c->half_v = c->blocks_v;
@@ -819,7 +841,7 @@ int build_wave(dg_gpu_ctx* c) {
     tmp.erase(std::unique(tmp.begin(), tmp.end()), tmp.end());
     for (int k : tmp) nlist.push_back(k);
     nstart[u + 1] = (int)nlist.size();
-    Lb = std::max(Lb, tmp.back() / WPB - u / WPB);
+    Lb = std::max({Lb, tmp.back() / WPB - u / WPB, u / WPB - tmp.front() / WPB});
     W = std::max(W, (int)tmp.size());
   }
   if (W > 32) return fail(DG_ERR_UNSUPPORTED, "wavefront wait list longer than a warp");
@@ -870,6 +892,7 @@ int build_wave(dg_gpu_ctx* c) {
   w.NU = NU;
   w.NB = NB;
   w.W = W;
+  w.back = larger_than_l2(c);
   // margin over the bandwidth, in blocks: 10 warps per SM (about 60 % of the resident warps),
   // so that the velocity updates a stress update needs have mostly finished when it starts,
   // while the lag window stays in L2; measured flat from 1,200 to 1,800 warps on the 200k-element

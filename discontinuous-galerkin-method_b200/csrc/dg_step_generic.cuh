@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(256, 2) k_stress(const __grid_constant__ Ops<R
   const long long t = ctr->s;
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->v = t + 1;
   if (t >= m.steps) return;
+  if (!MULTI) lb = stress_block(m, lb);
   if (lb >= m.n_elem_blocks) { record(m, lb - m.n_elem_blocks, t); return; }
   stress_body<A, KAHAN>(ops, m, lb, t);
 }

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(256, 1) k_stress_ref(const __grid_constant__ O
   const long long t = ctr->s;
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->v = t + 1;
   if (t >= m.steps) return;
+  if (!MULTI) lb = stress_block(m, lb);
   if (lb >= m.n_elem_blocks) { record(m, lb - m.n_elem_blocks, t); return; }
   const int S = m.S;
   const long long g = (long long)lb * blockDim.x + threadIdx.x;

@@ -34,6 +34,8 @@ struct Wave {
   int NB;                 // blocks of units: ceil(NU / warps per block)
   int L;                  // lag between a unit's velocity and its stress work, in blocks
   int W;                  // wait-list width (<= 32)
+  int back;               // odd steps take the blocks of units backwards: a step starts with the values
+                          // the one before it left in L2
   const int* wait;        // [NU][W] units holding the unit's elements or their neighbours, -1 padded
   unsigned int* vflag;    // [NU] step id (t + 1) once the unit's new velocities are stored
   const int* rec_start;   // [NU + 1] receivers whose element the unit covers:
@@ -172,15 +174,18 @@ __device__ __forceinline__ void wait_units(const Wave& w, int k, unsigned id) {
 }
 
 // The work of ticket tau in step t: the velocity half of the units of block tau and the stress
-// half of the units of block tau - L (each warp one unit of each).
+// half of the units of block tau - L (each warp one unit of each), counted from the last block
+// on odd steps where Wave::back says so (the lag covers the unit bandwidth both ways).
 template <class Layout, bool KAHAN>
 __device__ __forceinline__ void wave_ticket(const Ops2& ops, const MeshDev<float>& m, const Wave& w, int tau,
                                             long long t) {
   const unsigned id = (unsigned)(t + 1);
   const int wpb = (int)(blockDim.x >> 5), warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-  const int uv = tau * wpb + warp, j = tau - w.L, ut = j * wpb + warp;
-  const bool do_v = tau < w.NB && uv < w.NU;
-  const bool do_t = j >= 0 && j < w.NB && ut < w.NU;
+  const bool back = w.back && (t & 1);
+  const int bv = back ? w.NB - 1 - tau : tau, bt = back ? w.NB - 1 - (tau - w.L) : tau - w.L;
+  const int uv = bv * wpb + warp, ut = bt * wpb + warp;
+  const bool do_v = bv >= 0 && bv < w.NB && uv < w.NU;
+  const bool do_t = bt >= 0 && bt < w.NB && ut < w.NU;
   // the stress unit's wait list and the velocity unit's receiver range are fetched before the
   // velocity work, so their latency hides behind it
   const int k = (do_t && lane < w.W) ? __ldg(w.wait + (long long)ut * w.W + lane) : -1;
@@ -190,13 +195,13 @@ __device__ __forceinline__ void wave_ticket(const Ops2& ops, const MeshDev<float
     r1 = __ldg(w.rec_start + uv + 1);
   }
   if (do_v) {
-    Layout::template velocity<KAHAN>(ops, m, tau, t);
+    Layout::template velocity<KAHAN>(ops, m, bv, t);
     __syncwarp();
     if (r0 != r1) Layout::record(m, w, uv, r0, r1, t);
     __syncwarp();
   }
   typename Layout::Pre pre{};
-  if (do_t) pre = Layout::prefetch(m, j);
+  if (do_t) pre = Layout::prefetch(m, bt);
   // the warp barrier above orders every lane's stores before lane 0's release (a release fence
   // and a relaxed store: 0.6103 against 0.6112 ms a step with st.release on the 200k x 64 batch)
   if (do_v && lane == 0) {
@@ -205,7 +210,7 @@ __device__ __forceinline__ void wave_ticket(const Ops2& ops, const MeshDev<float
   }
   if (do_t) {
     wait_units(w, k, id);
-    Layout::template stress<KAHAN>(ops, m, j, t, pre);
+    Layout::template stress<KAHAN>(ops, m, bt, t, pre);
   }
 }
 

@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256, 2) k_stress_x2(const __grid_constant__ Op
   const long long t = ctr->s;
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->v = t + 1;
   if (t >= m.steps) return;
-  const int lb = blockIdx.x + m.block0;
+  const int lb = stress_block(m, blockIdx.x + m.block0);
   if (lb >= m.n_elem_blocks) { record(m, lb - m.n_elem_blocks, t); return; }
   stress_x2_body<S, KAHAN, false, PM>(ops, m, lb, t);
 }
@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(256, 2) k_stress_x2e(const __grid_constant__ O
   const long long t = ctr->s;
   if (threadIdx.x == 0 && blockIdx.x == 0) ctr->v = t + 1;
   if (t >= m.steps) return;
-  const int lb = blockIdx.x + m.block0;
+  const int lb = stress_block(m, blockIdx.x + m.block0);
   if (lb >= m.n_elem_blocks) { record(m, lb - m.n_elem_blocks, t); return; }
   stress_x2e_body<KAHAN>(ops, m, lb, t);
 }
