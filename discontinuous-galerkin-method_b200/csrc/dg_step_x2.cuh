@@ -598,8 +598,11 @@ __device__ __forceinline__ void velocity_x2e_body(const Ops2& ops, const MeshDev
   }
 }
 
+// Registers: 168 a thread (12 warps an SM) hold a face's gathers of both elements and the old values in
+// flight together; 128 (16 warps) run 9 % slower on the velocity half (us: 388,000 elements 22.9 -> 20.9,
+// 2 M Kahan 133.5 -> 121.2), 144 and 200 in between.
 template <bool KAHAN>
-__global__ void __launch_bounds__(256, 2) k_velocity_x2e(const __grid_constant__ Ops2 ops,
+__global__ void __maxnreg__(168) k_velocity_x2e(const __grid_constant__ Ops2 ops,
                                                          const __grid_constant__ MeshDev<float> m,
                                                          Counters* __restrict__ ctr) {
   pdl_enter();
@@ -714,8 +717,9 @@ __device__ __forceinline__ void stress_x2e_body(const Ops2& ops, const MeshDev<f
   }
 }
 
+// Registers: 128 a thread, for Kahan 112 (18 warps an SM; 2 M elements, us: 112 131, 128 142, 168 140).
 template <bool KAHAN>
-__global__ void __launch_bounds__(256, 2) k_stress_x2e(const __grid_constant__ Ops2 ops,
+__global__ void __maxnreg__(KAHAN ? 112 : 128) k_stress_x2e(const __grid_constant__ Ops2 ops,
                                                        const __grid_constant__ MeshDev<float> m,
                                                        Counters* __restrict__ ctr) {
   pdl_enter();
