@@ -156,6 +156,11 @@ struct dg_gpu_ctx {
   unsigned res_seq = 1;
   Resident rs{};
   int* res_error = nullptr;
+  // a batch of meshes stepped as one context per mesh, side by side: the contexts, the order in
+  // which a step call takes them (costliest first), the fork event of a call
+  std::vector<std::unique_ptr<dg_gpu_ctx>> subs;
+  std::vector<int> sub_order;
+  cudaEvent_t ev_fork = nullptr;
   struct Halo {
     int* d_send = nullptr;
     int* d_recv = nullptr;
@@ -229,6 +234,7 @@ struct dg_gpu_ctx {
     for (auto& e : ev_wave)
       if (e) cudaEventDestroy(e);
     if (wave_host) cudaFreeHost(wave_host);
+    if (ev_fork) cudaEventDestroy(ev_fork);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     for (void* p : allocs) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
@@ -1479,7 +1485,81 @@ const char* dg_gpu_strerror(int code) {
 
 const char* dg_gpu_last_error(void) { return g_last.c_str(); }
 
-int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts_in) {
+// dg_gpu_init; member: the context of one mesh of a batch (several step side by side, so none of them
+// takes a form whose blocks must all be resident at once)
+static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts, bool member);
+
+// Whether a batch is stepped mesh by mesh: the engine's own choice of kernels throughout, the
+// same operators for every mesh, no watchdog (it stops all meshes at the same step), and meshes of
+// 50,000 lanes on average, so that a mesh's launches keep the GPU busy while the host enqueues the
+// next (DG_BATCH_BY_MESH=0/1 overrides the size).  Each mesh then has the kernels of its own shot
+// count, its state in L2 for the whole call where it fits, and no mesh waits for the others' half
+// steps.  us a step against all meshes in each launch, calls of 50 steps and of one: 12 uneven
+// meshes FP32 388 -> 352 and 419 -> 398, Kahan 724 -> 567 and 750 -> 611, FP64 772 -> 729 and
+// 785 -> 775; 24 of 80,000 lanes 274 -> 184 and 301 -> 268; 8 of 57,600 68 -> 43 and 81 -> 78; below
+// the line 8 of 14,400 19 -> 22 and 31 -> 66, 12 of 20,000 FP64 42 -> 42 and 54 -> 94.  At most
+// 256 meshes: each has streams and graphs of its own.
+static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
+  const char* env = getenv("DG_BATCH_BY_MESH");
+  if (n < 2 || n > 256 || o.variant != 0 || o.wavefront == 1 || o.autotune || o.block_threads || o.watchdog_every > 0 ||
+      getenv("DG_MX_PERSISTENT") || (env && atoi(env) == 0))
+    return false;
+  double lanes = 0;
+  for (int k = 0; k < n; k++) {
+    if (!m[k].Vr || !m[k].Vs || !m[k].inverV || !m[k].S || m[k].K <= 0 || m[k].n_shots < 1) return false;
+    const double s = m[k].n_shots;
+    lanes += m[k].K * (o.precision <= DG_FP64 ? s : s / 2);
+    if (k && (memcmp(m[k].Vr, m[0].Vr, 36 * sizeof(double)) || memcmp(m[k].Vs, m[0].Vs, 36 * sizeof(double)) ||
+              memcmp(m[k].inverV, m[0].inverV, 36 * sizeof(double)) || memcmp(m[k].S, m[0].S, 54 * sizeof(double))))
+      return false;
+  }
+  return env ? true : lanes >= 50000.0 * n;
+}
+
+static int init_subs(dg_gpu_ctx* c, const dg_gpu_mesh* meshes, int n, const dg_gpu_opts& o) {
+  dg_gpu_opts so = o;
+  so.wavefront = -1;  // as in a batch: half steps stay possible
+  if (so.graph_steps == 0) so.graph_steps = 24;  // 100 a graph: 2 ms more a mesh here, the same steps
+  c->mi.assign(n, MeshHostInfo());
+  c->stats.dof_per_step = 0;
+  c->bytes_two_pass = 0;
+  std::vector<double> cost(n);
+  for (int k = 0; k < n; k++) {
+    dg_gpu_ctx* sub = nullptr;
+    int rc = init_context(&sub, &meshes[k], 1, &so, true);
+    if (rc) return rc;
+    c->subs.emplace_back(sub);
+    c->mi[k].K = sub->mi[0].K;
+    c->mi[k].S = sub->mi[0].S;
+    c->mi[k].n_rec = sub->mi[0].n_rec;
+    c->mi[k].steps = sub->mi[0].steps;
+    c->max_steps = std::max(c->max_steps, sub->max_steps);
+    c->stats.dof_per_step += sub->stats.dof_per_step;
+    c->bytes_two_pass += sub->bytes_two_pass;
+    cost[k] = (double)sub->mi[0].K * sub->mi[0].S_pad;
+    c->sub_order.push_back(k);
+  }
+  std::stable_sort(c->sub_order.begin(), c->sub_order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+  CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+  c->block = c->subs[0]->block;
+  c->graph_steps = c->subs[0]->graph_steps;
+  return DG_OK;
+}
+
+// Orders a mesh's stream after the context's, and back: around the calls that work on one mesh.
+static int sub_begin(dg_gpu_ctx* c, dg_gpu_ctx* sub) {
+  CK(cudaEventRecord(c->ev_fork, c->stream));
+  CK(cudaStreamWaitEvent(sub->stream, c->ev_fork, 0));
+  return DG_OK;
+}
+static int sub_end(dg_gpu_ctx* c, dg_gpu_ctx* sub) {
+  CK(cudaEventRecord(c->ev_fork, sub->stream));
+  CK(cudaStreamWaitEvent(c->stream, c->ev_fork, 0));
+  return DG_OK;
+}
+
+static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts_in,
+                        bool member) {
   if (!out) return fail(DG_ERR_ARG, "ctx pointer is null");
   *out = nullptr;
   if (!meshes || n_meshes < 1) return fail(DG_ERR_ARG, "need at least one mesh");
@@ -1493,14 +1573,15 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= o.device || o.device < 0)
     return fail(DG_ERR_NODEVICE, "no CUDA device with that ordinal");
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, o.device));
-  if (prop.major != 10) return fail(DG_ERR_NODEVICE, "the engine is built for sm_100a (B200)");
+  int major = 0, sms = 0;  // two attributes: the whole property record takes milliseconds
+  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, o.device));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, o.device));
+  if (major != 10) return fail(DG_ERR_NODEVICE, "the engine is built for sm_100a (B200)");
   CK(cudaSetDevice(o.device));
 
   std::unique_ptr<dg_gpu_ctx> c(new dg_gpu_ctx());
   c->device = o.device;
-  c->num_sms = prop.multiProcessorCount;
+  c->num_sms = sms;
   c->precision = o.precision;
   c->is_double = o.precision == DG_FP64_REF || o.precision == DG_FP64;
   c->kahan = o.precision == DG_FP32_KAHAN;
@@ -1516,6 +1597,16 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   CK(cudaEventCreateWithFlags(&c->ev_wavelet, cudaEventDisableTiming));
   for (auto& e : c->ev) CK(cudaEventCreate(&e));
 
+  if (batch_by_mesh(meshes, n_meshes, o)) {
+    const int rc = init_subs(c.get(), meshes, n_meshes, o);
+    if (rc == DG_OK) {
+      *out = c.release();
+      return DG_OK;
+    }
+    c->subs.clear();  // no room for a context per mesh, or input that the checks below report
+    cudaGetLastError();
+  }
+  c->mi.clear();
   c->mi.resize(n_meshes);
   double bytes = 0, dof = 0;
   size_t stage = 1, trace_chunk = 0;
@@ -1676,7 +1767,7 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   }
   if (o.autotune && !o.block_threads)
     if ((rc = autotune(c.get(), o.tune_cache))) return rc;
-  if ((rc = build_resident(c.get()))) return rc;
+  if (!member && (rc = build_resident(c.get()))) return rc;
   c->graph_steps = o.graph_steps < 0 ? 0 : (o.graph_steps ? o.graph_steps : (int)std::min<long>(100, c->max_steps));
   if ((rc = rebuild_graph(c.get()))) return rc;
   if ((rc = zero_state(c.get()))) return rc;
@@ -1684,6 +1775,10 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   c->stats.graph_steps = c->graph_steps;
   *out = c.release();
   return DG_OK;
+}
+
+int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts) {
+  return init_context(out, meshes, n_meshes, opts, false);
 }
 
 // Enqueue n steps on the context stream (graphs where they fit; the watchdog, when on,
@@ -1789,12 +1884,104 @@ static int steps_done_event(dg_gpu_ctx* c, long t, cudaEvent_t* out) {
   return DG_OK;
 }
 
+// n steps of every mesh of a batch stepped mesh by mesh, forked from and joined to the context
+// stream.  A mesh takes all its steps before the next of its chain.  First, one at a time, the
+// meshes whose state is well past L2 (they run at HBM rate alone, and would push the others' state
+// out of L2), then the others in chains side by side (12 uneven meshes, us a step in calls of 50
+// and of one: one chain 384 and 510, two 373 and 480, two after the large mesh 353 and 435, four
+// after it 353 and 405).
+static int enqueue_subs(dg_gpu_ctx* c, long n) {
+  constexpr int kChains = 4;
+  constexpr double kAlone = 150e6;  // bytes of state
+  const auto bytes = [&](int k) {
+    return 30.0 * (c->is_double ? 8 : 4) * (c->kahan ? 2 : 1) * c->subs[k]->mi[0].K * c->subs[k]->mi[0].S_pad;
+  };
+  // in a call of many steps no more chains than keep their states in L2 together (4 meshes of
+  // 28,800 elements, 8 shots, 28 MB each: two chains 43.1 us a step, four 62.2); in a short one
+  // the gaps between launches cost more (24 meshes of 20,000, 8 shots, 5 steps a call: 265, 231)
+  int chains = kChains;
+  if (n >= 16) {
+    double held = 0;
+    chains = 0;
+    for (int k : c->sub_order)
+      if (bytes(k) <= kAlone && chains < kChains && (held += bytes(k)) <= 75e6) chains++;
+    chains = std::max(chains, 2);
+  }
+  CK(cudaEventRecord(c->ev_fork, c->stream));
+  cudaEvent_t last[kChains];
+  double load[kChains] = {};
+  std::fill(last, last + kChains, c->ev_fork);
+  c->stats.launches = 0;
+  for (int k : c->sub_order) {  // costliest first
+    dg_gpu_ctx* sub = c->subs[k].get();
+    const long m = std::min(n, sub->max_steps - sub->t);
+    if (m <= 0) continue;  // past its last step
+    const double lanes = (double)sub->mi[0].K * sub->mi[0].S_pad;
+    const bool alone = bytes(k) > kAlone;
+    const int at = (int)(std::min_element(load, load + chains) - load);
+    CK(cudaStreamWaitEvent(sub->stream, last[at], 0));
+    int rc = enqueue_steps(sub, m, false);
+    if (rc || (rc = mark_steps(sub))) return rc;
+    const cudaEvent_t done = sub->marks[(sub->mark_next + dg_gpu_ctx::kMarks - 1) % dg_gpu_ctx::kMarks].ev;
+    if (alone) {
+      std::fill(last, last + kChains, done);
+    } else {
+      last[at] = done;
+      load[at] += lanes * m;
+    }
+    c->stats.launches += sub->stats.launches;
+  }
+  for (cudaEvent_t e : last) CK(cudaStreamWaitEvent(c->stream, e, 0));
+  c->t += n;
+  c->stats.steps_done = c->t;
+  return DG_OK;
+}
+
+// The same with each step timed on the context stream (as the "velocity" interval).
+static int timed_subs(dg_gpu_ctx* c, long n, int flush_l2, float* ms, double* total) {
+  long launches = 0;
+  *total = 0;
+  for (long k = 0; k < n; k++) {
+    if (flush_l2) CK(cudaMemsetAsync(c->d_flush, (int)(k & 0xff), c->flush_bytes, c->stream));
+    CK(cudaEventRecord(c->ev[0], c->stream));
+    int rc = enqueue_subs(c, 1);
+    if (rc) return rc;
+    launches += c->stats.launches;
+    CK(cudaEventRecord(c->ev[1], c->stream));
+    CK(cudaEventSynchronize(c->ev[1]));
+    float t = 0;
+    CK(cudaEventElapsedTime(&t, c->ev[0], c->ev[1]));
+    if (ms) ms[k] = t;
+    *total += t;
+  }
+  c->stats.launches = launches;
+  c->stats.ms_velocity = *total;
+  c->stats.ms_stress = 0;
+  return DG_OK;
+}
+
+static int check_subs(dg_gpu_ctx* c) {
+  int bad = DG_OK;
+  for (auto& sub : c->subs) {
+    const int rc = check_wave(sub.get());
+    if (rc) bad = rc;
+  }
+  return bad;
+}
+
 static int do_steps(dg_gpu_ctx* c, long n, bool timed, bool wait = true) {
   if (!c || n < 0) return fail(DG_ERR_ARG, "bad arguments");
   if (c->half_pending || c->part_done)
     return fail(DG_ERR_STATE, "a half step is waiting for its other half or part");
   if (c->t + n > c->max_steps) return fail(DG_ERR_STATE, "stepping past the end of the wavelet table");
   CK(cudaSetDevice(c->device));
+  if (!c->subs.empty()) {
+    double total = 0;
+    const int rc = timed ? timed_subs(c, n, 0, nullptr, &total) : enqueue_subs(c, n);
+    if (rc || !wait) return rc;
+    CK(cudaStreamSynchronize(c->stream));
+    return check_subs(c);
+  }
   int rc = enqueue_steps(c, n, timed);
   if (rc) return rc;
   if ((rc = mark_steps(c))) return rc;
@@ -1810,6 +1997,10 @@ int dg_gpu_synchronize(dg_gpu_ctx* c) {
   if (!c) return fail(DG_ERR_ARG, "null context");
   CK(cudaSetDevice(c->device));
   CK(cudaStreamSynchronize(c->stream));
+  if (!c->subs.empty()) {
+    for (auto& sub : c->subs) CK(cudaStreamSynchronize(sub->stream));
+    return check_subs(c);
+  }
   return check_wave(c);
 }
 int dg_gpu_step_timed(dg_gpu_ctx* c, long n) { return do_steps(c, n, true); }
@@ -1843,6 +2034,13 @@ int dg_gpu_step_profiled(dg_gpu_ctx* c, long n, int flush_l2, float* ms_vel, flo
   CK(cudaSetDevice(c->device));
   int rc;
   if (flush_l2 && (rc = ensure_flush(c))) return rc;
+  if (!c->subs.empty()) {
+    double total = 0;
+    if ((rc = timed_subs(c, n, flush_l2, ms_vel, &total))) return rc;
+    if (ms_str) std::fill(ms_str, ms_str + n, 0.f);
+    if (ms_total) *ms_total = total;
+    return check_subs(c);
+  }
   std::vector<cudaEvent_t> ev((size_t)3 * n);
   for (auto& e : ev) CK(cudaEventCreate(&e));
   for (long k = 0; k < n; k++) {
@@ -1877,7 +2075,8 @@ int dg_gpu_step_profiled(dg_gpu_ctx* c, long n, int flush_l2, float* ms_vel, flo
   return check_wave(c);
 }
 
-int dg_gpu_fetch_traces(dg_gpu_ctx* c, int mesh, long t0, long n, double* dst_x, double* dst_z) {
+// dg_gpu_fetch_traces but for the wait: the copies are enqueued on the copy stream
+static int fetch_traces_enqueue(dg_gpu_ctx* c, int mesh, long t0, long n, double* dst_x, double* dst_z) {
   if (!c || !dst_x || !dst_z || mesh < DG_ALL_MESHES || mesh >= (int)c->mi.size() || t0 < 0 || n < 0)
     return fail(DG_ERR_ARG, "bad arguments");
   // the meshes asked for, their blocks one after the other in both outputs
@@ -1916,7 +2115,29 @@ int dg_gpu_fetch_traces(dg_gpu_ctx* c, int mesh, long t0, long n, double* dst_x,
   }
   CK(cudaMemcpyAsync(dst_x, c->d_stage, total * sizeof(double), cudaMemcpyDeviceToHost, cs));
   CK(cudaMemcpyAsync(dst_z, c->d_stage + total, total * sizeof(double), cudaMemcpyDeviceToHost, cs));
-  CK(cudaStreamSynchronize(cs));
+  return DG_OK;
+}
+
+int dg_gpu_fetch_traces(dg_gpu_ctx* c, int mesh, long t0, long n, double* dst_x, double* dst_z) {
+  if (!c || c->subs.empty()) {
+    const int rc = fetch_traces_enqueue(c, mesh, t0, n, dst_x, dst_z);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(c->copy_stream));
+    return DG_OK;
+  }
+  if (!dst_x || !dst_z || mesh < DG_ALL_MESHES || mesh >= (int)c->mi.size() || t0 < 0 || n < 0)
+    return fail(DG_ERR_ARG, "bad arguments");
+  const int k0 = mesh == DG_ALL_MESHES ? 0 : mesh, k1 = mesh == DG_ALL_MESHES ? (int)c->mi.size() : mesh + 1;
+  for (int k = k0; k < k1; k++)
+    if (t0 + n > std::min(c->t, c->mi[k].steps)) return fail(DG_ERR_STATE, "trace window beyond the steps taken");
+  CK(cudaSetDevice(c->device));
+  long long at = 0;
+  for (int k = k0; k < k1; k++) {
+    const int rc = fetch_traces_enqueue(c->subs[k].get(), 0, t0, n, dst_x + at, dst_z + at);
+    if (rc) return rc;
+    at += (long long)n * c->mi[k].n_rec * c->mi[k].S;
+  }
+  for (int k = k0; k < k1; k++) CK(cudaStreamSynchronize(c->subs[k]->copy_stream));
   return DG_OK;
 }
 
@@ -1945,6 +2166,11 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
   if (shot < 0 || shot >= h.S) return fail(DG_ERR_ARG, "shot out of range");
   if (c->t + n > c->max_steps) return fail(DG_ERR_STATE, "stepping past the end of the wavelet table");
   CK(cudaSetDevice(c->device));
+  dg_gpu_ctx* const all = c;  // steps every mesh; c from here on: the context that holds this one
+  if (!c->subs.empty()) {
+    c = c->subs[mesh].get();
+    mesh = 0;
+  }
   const size_t per = (size_t)h.K * 6;  // doubles per field
   if (per > c->snap_elems) {            // (re)size the rings: 2 slots x (Vx, Vz)
     if (c->snap_host) {
@@ -1966,7 +2192,7 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
     }
   }
   const long J = n / every;
-  const long t0 = c->t;
+  const long t0 = all->t;
   auto deliver = [&](long j) -> int {
     const int slot = (int)(j & 1);
     CK(cudaEventSynchronize(c->snap_copy[slot]));
@@ -1977,7 +2203,7 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
   int rc;
   for (long j = 0; j < J; j++) {
     const int slot = (int)(j & 1);
-    if ((rc = enqueue_steps(c, every, false))) return rc;
+    if ((rc = all == c ? enqueue_steps(c, every, false) : enqueue_subs(all, every))) return rc;
     // the device slot is free once the copy of snapshot j - 2 has finished
     if (j >= 2) CK(cudaStreamWaitEvent(c->stream, c->snap_copy[slot], 0));
     double* dslot = c->snap_dev + (size_t)slot * 2 * c->snap_elems;
@@ -1993,12 +2219,17 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
   }
   if (J >= 1 && (rc = deliver(J - 1))) return rc;
   CK(cudaStreamSynchronize(c->stream));
+  if (all != c) {
+    CK(cudaStreamSynchronize(all->stream));
+    return check_subs(all);
+  }
   c->stats.steps_done = c->t;
   return check_wave(c);
 }
 
 int dg_gpu_fetch(dg_gpu_ctx* c, int what, int mesh, int shot, double* dst) {
   if (!c || !dst || mesh < 0 || mesh >= (int)c->mi.size()) return fail(DG_ERR_ARG, "bad arguments");
+  if (!c->subs.empty()) return dg_gpu_fetch(c->subs[mesh].get(), what, 0, shot, dst);
   const MeshHostInfo& h = c->mi[mesh];
   const bool all = shot == DG_ALL_SHOTS && what >= DG_VX && what <= DG_TXZ;
   if (!all && (shot < 0 || shot >= h.S)) return fail(DG_ERR_ARG, "shot out of range");
@@ -2055,6 +2286,7 @@ int dg_gpu_fetch(dg_gpu_ctx* c, int what, int mesh, int shot, double* dst) {
 
 int dg_gpu_load(dg_gpu_ctx* c, int what, int mesh, int shot, const double* src) {
   if (!c || !src || mesh < 0 || mesh >= (int)c->mi.size()) return fail(DG_ERR_ARG, "bad arguments");
+  if (!c->subs.empty()) return dg_gpu_load(c->subs[mesh].get(), what, 0, shot, src);
   const MeshHostInfo& h = c->mi[mesh];
   if (shot < 0 || shot >= h.S) return fail(DG_ERR_ARG, "shot out of range");
   if (what < DG_VX || what > DG_TXZ) return fail(DG_ERR_STATE, "only fields can be loaded");
@@ -2080,6 +2312,15 @@ int dg_gpu_reset(dg_gpu_ctx* c) {
   CK(cudaSetDevice(c->device));
   c->half_pending = false;
   c->part_done = 0;
+  if (!c->subs.empty()) {
+    CK(cudaStreamSynchronize(c->stream));
+    for (auto& sub : c->subs) {
+      const int rc = dg_gpu_reset(sub.get());
+      if (rc) return rc;
+    }
+    c->t = 0;
+    return DG_OK;
+  }
   return zero_state(c);
 }
 
@@ -2091,7 +2332,12 @@ int dg_gpu_half_step(dg_gpu_ctx* c, int half) {
     return fail(DG_ERR_STATE, half == 0 ? "velocity half again before the stress half" : "stress half without the velocity half");
   if (half == 0 && c->t + 1 > c->max_steps) return fail(DG_ERR_STATE, "stepping past the end of the wavelet table");
   CK(cudaSetDevice(c->device));
-  int rc = launch_step(c, nullptr, nullptr, nullptr, half == 0 ? 1 : 2);
+  int rc = DG_OK;
+  if (c->subs.empty()) rc = launch_step(c, nullptr, nullptr, nullptr, half == 0 ? 1 : 2);
+  for (auto& sub : c->subs) {
+    if (half == 0 ? sub->t >= sub->max_steps : !sub->half_pending) continue;  // past its last step
+    if ((rc = sub_begin(c, sub.get())) || (rc = dg_gpu_half_step(sub.get(), half)) || (rc = sub_end(c, sub.get()))) break;
+  }
   if (rc) return rc;
   c->half_pending = half == 0;
   if (half == 1) {
@@ -2174,6 +2420,7 @@ int dg_gpu_halo_lists(dg_gpu_ctx* c, int mesh, long n_send, const long* send, lo
   if (!c || mesh < 0 || mesh >= (int)c->mi.size() || n_send < 0 || n_recv < 0 || (n_send && !send) ||
       (n_recv && !recv))
     return fail(DG_ERR_ARG, "bad arguments");
+  if (!c->subs.empty()) return dg_gpu_halo_lists(c->subs[mesh].get(), 0, n_send, send, n_recv, recv);
   const MeshHostInfo& h = c->mi[mesh];
   std::vector<int> a(n_send), b(n_recv);
   for (long k = 0; k < n_send; k++) {
@@ -2220,6 +2467,13 @@ int dg_gpu_halo_lists(dg_gpu_ctx* c, int mesh, long n_send, const long* send, lo
 static int halo_copy(dg_gpu_ctx* c, int mesh, int what, void* buf, bool pack, bool sync = true) {
   if (!c || mesh < 0 || mesh >= (int)c->mi.size() || (what != 0 && what != 1))
     return fail(DG_ERR_ARG, "bad arguments");
+  if (!c->subs.empty()) {
+    CK(cudaSetDevice(c->device));
+    dg_gpu_ctx* sub = c->subs[mesh].get();
+    int rc = sub_begin(c, sub);
+    if (rc || (rc = halo_copy(sub, 0, what, buf, pack, sync))) return rc;
+    return sub_end(c, sub);
+  }
   if ((int)c->halo.size() <= mesh) return fail(DG_ERR_STATE, "no halo lists for this mesh");
   const dg_gpu_ctx::Halo& hl = c->halo[mesh];
   const long n = pack ? hl.n_send : hl.n_recv;
@@ -2290,6 +2544,13 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   for (int k = k0; k < k1; k++)
     if (t0 + n > c->mi[k].steps) return fail(DG_ERR_ARG, "wavelet window beyond a mesh's steps");
   CK(cudaSetDevice(c->device));
+  if (!c->subs.empty()) {
+    for (int k = k0; k < k1; k++) {
+      const int rc = dg_gpu_set_wavelet(c->subs[k].get(), 0, t0, n, w + (size_t)(k - k0) * n);
+      if (rc) return rc;
+    }
+    return DG_OK;
+  }
   // a few samples (a driver that sends each step's): through the staging buffer on the context
   // stream, behind the steps enqueued and ahead of the next, without a wait (1.8 us a call against
   // 8 with the copy stream, its event and the wait)
@@ -2357,6 +2618,7 @@ int dg_gpu_stats_get(dg_gpu_ctx* c, dg_gpu_stats* out) {
           : (c->wave ? (c->wave_persistent ? 6 : 5)
                      : (c->mx ? (c->mx_persistent ? 8 : 4)
                               : (c->gen_p2 ? 1 : (c->x2 == 1 ? 3 : (c->x2 ? (c->x2pm ? 7 : 2) : 1)))));
+  if (!c->subs.empty()) c->stats.kernel_family = 9;
   c->stats.bytes_per_step = c->wave ? c->bytes_wave : c->bytes_two_pass;
   *out = c->stats;
   return DG_OK;
@@ -2368,6 +2630,7 @@ int dg_gpu_free(dg_gpu_ctx* c) {
   if (!c) return DG_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
+  for (auto& sub : c->subs) cudaStreamSynchronize(sub->stream);
   delete c;
   return DG_OK;
 }

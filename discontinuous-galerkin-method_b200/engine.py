@@ -96,11 +96,14 @@ KERNEL_FAMILIES = {0: "reference operators (k_velocity_ref/k_stress_ref)",
                       "per thread, L2-resident lag (k_step_wave_p)",
                    7: "two shots per thread, packed FP32x2, plane-major layout (k_velocity_x2/k_stress_x2)",
                    8: "batch of meshes in one persistent cooperative launch, grid barrier between the halves "
-                      "(k_step_mx_p)"}
+                      "(k_step_mx_p)",
+                   9: "batch of meshes, each with the kernels of a mesh of its own (1, 2, 3, 7 or, FP64_REF, 0), "
+                      "several meshes side by side"}
 KERNEL_NAMES = {0: ("k_velocity_ref", "k_stress_ref"), 1: ("k_velocity", "k_stress"),
                 2: ("k_velocity_x2", "k_stress_x2"), 3: ("k_velocity_x2e", "k_stress_x2e"),
                 4: ("k_velocity_mx", "k_stress_mx"), 5: ("k_step_wave", None),
-                6: ("k_step_wave_p", None), 7: ("k_velocity_x2", "k_stress_x2"), 8: ("k_step_mx_p", None)}
+                6: ("k_step_wave_p", None), 7: ("k_velocity_x2", "k_stress_x2"), 8: ("k_step_mx_p", None),
+                9: ("k_velocity/k_stress of each mesh", None)}
 
 
 _LIB = None
