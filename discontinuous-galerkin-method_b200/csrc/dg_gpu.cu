@@ -899,10 +899,11 @@ int build_wave(dg_gpu_ctx* c) {
   w.NB = NB;
   w.W = W;
   w.back = larger_than_l2(c);
-  // margin over the bandwidth, in blocks: 10 warps per SM (about 60 % of the resident warps),
+  // margin over the bandwidth, in blocks: 12 warps per SM (three quarters of the resident warps),
   // so that the velocity updates a stress update needs have mostly finished when it starts,
   // while the lag window stays in L2; measured flat from 1,200 to 1,800 warps on the 200k-element
-  // batch, much slower below 1,000 (DG_WAVE_MARGIN overrides it, in blocks, for tuning)
+  // batch, much slower below 1,000 (49,400 x 24, us a step: 150 warps 117, 450 104, 740 85,
+  // 1,000 80) (DG_WAVE_MARGIN overrides it, in blocks, for tuning)
   int margin = (c->num_sms * c->margin_warps_per_sm + WPB - 1) / WPB;
   if (const char* env = getenv("DG_WAVE_MARGIN")) margin = std::max(0, atoi(env));
   w.L = Lb + margin;
@@ -1497,11 +1498,10 @@ static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshe
 // steps.  us a step against all meshes in each launch, calls of 50 steps and of one: 12 uneven
 // meshes FP32 388 -> 352 and 419 -> 398, Kahan 724 -> 567 and 750 -> 611, FP64 772 -> 729 and
 // 785 -> 775; 24 of 80,000 lanes 274 -> 184 and 301 -> 268; 8 of 57,600 68 -> 43 and 81 -> 78; below
-// the line 8 of 14,400 19 -> 22 and 31 -> 66, 12 of 20,000 FP64 42 -> 42 and 54 -> 94.  At most
-// 256 meshes: each has streams and graphs of its own.
+// the line 8 of 14,400 19 -> 22 and 31 -> 66, 12 of 20,000 FP64 42 -> 42 and 54 -> 94.
 static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
   const char* env = getenv("DG_BATCH_BY_MESH");
-  if (n < 2 || n > 256 || o.variant != 0 || o.wavefront == 1 || o.autotune || o.block_threads || o.watchdog_every > 0 ||
+  if (n < 2 || o.variant != 0 || o.wavefront == 1 || o.autotune || o.block_threads || o.watchdog_every > 0 ||
       getenv("DG_MX_PERSISTENT") || (env && atoi(env) == 0))
     return false;
   double lanes = 0;
@@ -1645,8 +1645,8 @@ static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshe
         c->gen_p2 = true;
       }
     }
-    // the wavefront step: one FP32 mesh on the two-shot kernels; automatic = on
-    // automatic: from 16 shots on.  Below, a warp covers several elements and the scattered
+    // the wavefront step: one FP32 mesh on the two-shot kernels; automatic: from 16 shots on
+    // (and from wave_min on, below).  Below, a warp covers several elements and the scattered
     // small gathers in RCM order cost more than the HBM traffic the step saves (200k elements:
     // 2 shots 0.096 ms against 0.073 for two launches, 4 shots 0.103 against 0.091, 8 even,
     // 16 shots 0.199 against 0.228; one shot on 2M elements 0.234 against 0.185)
@@ -1786,6 +1786,12 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
 static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
   c->stats.launches = 0;
   if (timed) { c->stats.ms_velocity = 0; c->stats.ms_stress = 0; }
+  // a caller that captures the context stream gets plain launches: they take the step from the
+  // device's counters, so the capture can be replayed, which the resident step's tags forbid, and
+  // a graph cannot be launched into a capture
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(c->stream, &cap));
+  const bool plain = cap != cudaStreamCaptureStatusNone;
   long done = 0;
   while (done < n) {
     long chunk = n - done;
@@ -1805,7 +1811,7 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
         c->stats.ms_stress += b;
       }
       c->stats.launches += (c->wave || c->mx_persistent ? 1 : 2) * chunk;
-    } else if (c->resident) {
+    } else if (c->resident && !plain) {
       chunk = std::min<long>(chunk, 1L << 16);
       int rc = launch_resident(c, (int)chunk);
       if (rc) return rc;
@@ -1816,9 +1822,9 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
       c->stats.launches += 1;
     } else {
       long k = 0;
-      if (c->graph && c->graph_steps > 0)
+      if (c->graph && c->graph_steps > 0 && !plain)
         for (; k + c->graph_steps <= chunk; k += c->graph_steps) CK(cudaGraphLaunch(c->graph, c->stream));
-      if (c->graph_small && c->graph_small_steps > 0)
+      if (c->graph_small && c->graph_small_steps > 0 && !plain)
         for (; k + c->graph_small_steps <= chunk; k += c->graph_small_steps)
           CK(cudaGraphLaunch(c->graph_small, c->stream));
       for (; k < chunk; k++) {
