@@ -34,7 +34,7 @@ extern "C" {
 #define DG_ERR_UNSUPPORTED -7  /* Np != 6, Nfp != 3, more meshes than supported */
 #define DG_ERR_NODEVICE -8     /* no CUDA device, or not an sm_100 device */
 #define DG_ERR_ORIENTATION -9  /* a triangle with non-positive Jacobian (compact paths need CCW) */
-#define DG_ERR_TIMEOUT -10     /* a wait between blocks (wavefront step, grid barrier of a persistent batch) reached its limit */
+#define DG_ERR_TIMEOUT -10     /* a wait between blocks (wavefront step, small meshes' step, grid barrier of a persistent batch) reached its limit */
 
 /* arithmetic of the time loop */
 #define DG_FP64_REF 0    /* the reference's per-element Dx/Dz/Q/A/B arrays, its operation order,
@@ -93,7 +93,8 @@ typedef struct {
 	int reorder;         /* 1: renumber elements along a Hilbert curve of centroids for locality */
 	int block_threads;   /* threads per block, 0: automatic (or autotuned) */
 	int graph_steps;     /* steps per captured CUDA graph (plus one of a quarter of them for shorter
-	                        calls), 0: automatic (100), <0: no graphs */
+	                        calls), 0: automatic (100; 24 where a batch steps mesh by mesh), <0: no
+	                        graphs (the forms that loop over steps in one launch use none) */
 	int autotune;        /* 1: time candidate block sizes (and, for a batch of meshes, the persistent or
 	                        two-launch step; for the wavefront step its persistent form and lag) at init */
 	int watchdog_every;  /* check the velocity fields for NaN/Inf every k steps (0: off) */
@@ -101,8 +102,10 @@ typedef struct {
 	int variant;         /* FP32 kernels: 0 automatic, 1 one (element, shot) per thread,
 	                        2 packed FP32x2 kernels (two elements or two shots per thread; element-major
 	                        state for two shots per thread), 3 the same with plane-major state for 2-16 shots */
-	int wavefront;       /* one launch per step that keeps the state in flight in L2 (single FP32 mesh
-	                        of 1, 2, 4, ..., 128 shots): 0 automatic (on from 16 shots), 1 on, -1 off */
+	int wavefront;       /* one launch per step that keeps the state in flight in L2 (single FP32 mesh):
+	                        0 automatic (16 to 128 shots where the state does not stay in L2: from
+	                        1,000,000 elements x shots on, 250,000 in compensated FP32 with 17 to 127
+	                        shots that are no power of two), 1 on (1, 2, 4, ..., 128 shots), -1 off */
 } dg_gpu_opts;
 
 typedef struct {
@@ -122,7 +125,14 @@ typedef struct {
 	                          7 two shots per thread on plane-major state (FP32, 2-14 shots),
 	                          8 FP32 batch of meshes in one persistent cooperative launch for many steps,
 	                            the bodies of 4 with a grid barrier between the halves (default for
-	                            batches of at least 16 work blocks per resident block) */
+	                            batches of at least 16 work blocks per resident block),
+	                          9 batch of meshes, each stepped by a context of its own with the kernels of
+	                            a single mesh, several meshes side by side (default for batches of 50,000
+	                            lanes a mesh on average, a lane being one element and shot in FP64, one
+	                            and two shots in FP32).
+	                          A single mesh whose state fits in the SMs' registers runs dg_gpu_step in one
+	                          cooperative launch for all its steps; the family reported is then that of
+	                          its other calls (half steps, timed and profiled steps), with the same bits */
 } dg_gpu_stats;
 
 void dg_gpu_default_opts(dg_gpu_opts *opts);
@@ -151,7 +161,8 @@ int dg_gpu_step_timed(dg_gpu_ctx *ctx, long n);
 /* Advance n steps with a CUDA event before, between and after the two launches of every step,
  * all on the context stream and without host synchronisation until the end.  ms_vel / ms_str
  * (n floats each, may be NULL) receive each launch's device time (the wavefront step is one
- * launch: its time lands in ms_vel, ms_str holds about 0); ms_total the time from the
+ * launch, and a batch that steps mesh by mesh is timed step by step: the time lands in ms_vel,
+ * ms_str holds about 0); ms_total the time from the
  * first event to the last.  With flush_l2 != 0 a buffer larger than L2 is written before every
  * step, outside the timed launches (ms_total then counts launches only). */
 int dg_gpu_step_profiled(dg_gpu_ctx *ctx, long n, int flush_l2, float *ms_vel, float *ms_str, double *ms_total);
@@ -183,7 +194,8 @@ int dg_gpu_reset(dg_gpu_ctx *ctx);
  * w(t) on the host every step, DG_leap_Frog_OpenMP.c:421); mesh = DG_ALL_MESHES: w holds n
  * samples for each mesh, one after the other in mesh order.  Returns with w copied.  Steps
  * enqueued before the call that read these samples see the old ones; when none does (t0 at or
- * past the steps enqueued so far) the copy does not wait for the steps in flight. */
+ * past the steps enqueued so far) the copy does not wait for the steps in flight; up to 64
+ * samples are staged and copied in stream order without any wait. */
 int dg_gpu_set_wavelet(dg_gpu_ctx *ctx, int mesh, long t0, long n, const double *w);
 
 /* ---- one mesh split over several contexts (one per GPU): domain decomposition --------------
@@ -272,7 +284,7 @@ int dg_gpu_flush_l2(dg_gpu_ctx *ctx);
  * wrong; unit < 0 undoes it.  dg_gpu_reset then gives a context that steps as a fresh one.  On a
  * persistent batch of meshes (kernel family 8) unit >= 0 makes its grid barrier wait for one
  * block more than the grid holds, with a short limit (milliseconds), to the same effect.
- * DG_ERR_UNSUPPORTED when the context has neither. */
+ * DG_ERR_UNSUPPORTED when the context has neither (a batch that steps mesh by mesh waits nowhere). */
 int dg_gpu_debug_stall_wave(dg_gpu_ctx *ctx, int unit);
 
 /* Largest mesh dg_gpu_energy_noalloc accepts: its scratch holds one partial sum per 256 elements. */
