@@ -899,7 +899,7 @@ int build_wave(dg_gpu_ctx* c) {
   w.NB = NB;
   w.W = W;
   w.back = larger_than_l2(c);
-  // margin over the bandwidth, in blocks: 12 warps per SM (three quarters of the resident warps),
+  // margin over the bandwidth, in blocks: 12 or 14 warps per SM (of 16 resident ones),
   // so that the velocity updates a stress update needs have mostly finished when it starts,
   // while the lag window stays in L2; measured flat from 1,200 to 1,800 warps on the 200k-element
   // batch, much slower below 1,000 (49,400 x 24, us a step: 150 warps 117, 450 104, 740 85,
@@ -1423,7 +1423,7 @@ int autotune(dg_gpu_ctx* c, const char* cache) {
       continue;
     }
     for (int pers = c->wave_mid ? 1 : 0; pers < 2; pers++)
-      for (int mw : {8, 10, 14}) cand.push_back({b, pers, mw});
+      for (int mw : {10, 12, 14}) cand.push_back({b, pers, mw});
   }
   const long probe = std::min<long>(8, c->max_steps);
   float best = 1e30f;
@@ -1663,6 +1663,11 @@ static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshe
         c->no_halves = true;
       }
     }
+    // lag margin: smaller FP32 meshes take two warps per SM more (us a step at 12 / 14 / 16: 49,400
+    // x 24 75.4 / 73.2 / 73.4, 20,000 x 72 84.9 / 83.1 / 84.0, 180,000 x 16 166.5 / 165.6 / 166.8; but
+    // 320,000 x 24 437.9 / 438.6 / 441.7, 200,000 x 64 604 / 607 / 612, Kahan 28,800 x 48 132.7 / 133.1 /
+    // 135.5, 320,000 x 24 771 / 782 / 791)
+    if (c->wave && !c->kahan && (long long)meshes[k].K * meshes[k].n_shots < 4000000) c->margin_warps_per_sm = 14;
     if (o.wavefront == 1 && !c->wave)
       return fail(DG_ERR_UNSUPPORTED, "the wavefront step needs one FP32 mesh with 1, 2, 4, 8, ..., 128 shots");
     const char* arrays = getenv("DG_REF_ARRAYS");
