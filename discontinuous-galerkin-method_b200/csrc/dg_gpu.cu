@@ -1147,7 +1147,9 @@ int build_resident(dg_gpu_ctx* c) {
   c->res_blocks = nb;
   c->res_threads = (int)std::min<long>(max_threads, (w.nl + 31) / 32 * 32 + (most * H + 31) / 32 * 32);
   const void* kernel = resident_kernel(c);
-  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->res_smem));
+  // the limit belongs to the kernel, which other contexts of this process launch with other sizes:
+  // always the device's
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, c->res_threads, c->res_smem));
   if ((long)per_sm * c->num_sms < nb) return DG_OK;
