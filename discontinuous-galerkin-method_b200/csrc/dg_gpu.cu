@@ -214,6 +214,7 @@ struct dg_gpu_ctx {
   static constexpr int kWave = 256;  // doubles a half
   double* wave_host = nullptr;
   int wave_half = 0, wave_pos = 0;  // where the next update goes
+  long staged_end = 0;              // end of the samples whose copies may still be on their way
   cudaEvent_t ev_wave[2] = {nullptr, nullptr};
 
   ~dg_gpu_ctx() {
@@ -1371,6 +1372,7 @@ int zero_state(dg_gpu_ctx* c) {
   }
   CK(cudaStreamSynchronize(c->stream));
   c->t = 0;
+  c->staged_end = 0;
   for (auto& m : c->marks) m.t_end = -1;  // no step mark covers the new run's steps
   return DG_OK;
 }
@@ -2001,6 +2003,7 @@ static int do_steps(dg_gpu_ctx* c, long n, bool timed, bool wait = true) {
   c->stats.steps_done = c->t;
   if (!wait) return DG_OK;
   CK(cudaStreamSynchronize(c->stream));
+  c->staged_end = 0;
   return check_wave(c);
 }
 
@@ -2011,9 +2014,13 @@ int dg_gpu_synchronize(dg_gpu_ctx* c) {
   CK(cudaSetDevice(c->device));
   CK(cudaStreamSynchronize(c->stream));
   if (!c->subs.empty()) {
-    for (auto& sub : c->subs) CK(cudaStreamSynchronize(sub->stream));
+    for (auto& sub : c->subs) {
+      CK(cudaStreamSynchronize(sub->stream));
+      sub->staged_end = 0;
+    }
     return check_subs(c);
   }
+  c->staged_end = 0;
   return check_wave(c);
 }
 int dg_gpu_step_timed(dg_gpu_ctx* c, long n) { return do_steps(c, n, true); }
@@ -2584,6 +2591,7 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
     }
     double* const st = c->wave_host + c->wave_half * dg_gpu_ctx::kWave + c->wave_pos;
     c->wave_pos += (int)few;
+    c->staged_end = std::max(c->staged_end, t0 + n);
     memcpy(st, w, few * sizeof(double));
     for (int k = k0; k < k1; k++) {
       const double* dw = c->is_double ? c->md_d[k].wavelet : c->md_f[k].wavelet;
@@ -2593,8 +2601,9 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   }
   // samples that no enqueued step reads (t0 at or past the steps enqueued so far) go over the
   // copy stream, and the context stream waits for them, so steps in flight keep running;
-  // otherwise the copy follows the enqueued steps on the context stream
-  const bool ahead = t0 >= c->t;
+  // otherwise, and where a staged copy of an earlier call could still land on them, the copy
+  // follows the enqueued work on the context stream
+  const bool ahead = t0 >= c->t && t0 >= c->staged_end;
   int rc;
   if (ahead && ((rc = ensure_copy_stream(c)) || (rc = ensure_event(&c->ev_wavelet)))) return rc;
   cudaStream_t st = ahead ? c->copy_stream : c->stream;

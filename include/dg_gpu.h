@@ -195,7 +195,9 @@ int dg_gpu_reset(dg_gpu_ctx *ctx);
  * samples for each mesh, one after the other in mesh order.  Returns with w copied.  Steps
  * enqueued before the call that read these samples see the old ones; when none does (t0 at or
  * past the steps enqueued so far) the copy does not wait for the steps in flight; up to 64
- * samples are staged and copied in stream order without any wait. */
+ * samples are staged and copied in stream order without any wait, and a longer update that an
+ * earlier staged one may still overlap follows it there.  Of two updates of a sample the later
+ * call's stays. */
 int dg_gpu_set_wavelet(dg_gpu_ctx *ctx, int mesh, long t0, long n, const double *w);
 
 /* ---- one mesh split over several contexts (one per GPU): domain decomposition --------------

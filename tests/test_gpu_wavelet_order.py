@@ -1,0 +1,54 @@
+"""Wavelet updates take effect in the order of their calls, whichever way each travels: up to 64
+samples are staged and copied behind the steps enqueued, more go over the second stream ahead of
+them.
+"""
+import numpy as np
+import pytest
+
+from conftest import pkg
+
+eng = pkg.engine
+pytestmark = pytest.mark.gpu
+FIELDS = ("Vx", "Vz", "Txx", "Tzz", "Txz")
+LEAD, STEPS = 3000, 3300  # steps in flight while the updates are made, steps in all
+
+
+def _mesh(cells, shots):
+    m = eng.mesh_from_setup(pkg.host.build_setup(pkg.workloads.small_square(n_cells=cells, steps=STEPS, shots=shots), full=False),
+                            with_ref_ops=False)
+    m["wavelet"] = np.zeros(STEPS)
+    return m
+
+
+def _fields(e):
+    return [e.fetch(f, k, eng.ALL_SHOTS) for k in range(len(e.info)) for f in FIELDS]
+
+
+# (first sample, samples) of the updates, in the order they are made
+@pytest.mark.parametrize("updates", [((LEAD, 10), (LEAD, 200)), ((LEAD, 200), (LEAD + 5, 10)),
+                                     ((LEAD + 190, 30), (LEAD, 200)), ((LEAD, 64), (LEAD, 65), (LEAD + 3, 64)),
+                                     ((LEAD - 5, 20), (LEAD, 100)), ((LEAD, 30), (LEAD + 30, 100), (LEAD, 100))])
+@pytest.mark.parametrize("shapes", [((50, 1),), ((9, 1), (20, 4))])
+def test_the_last_update_of_a_sample_wins(updates, shapes, monkeypatch):
+    monkeypatch.setenv("DG_BATCH_BY_MESH", "1")
+    meshes = [_mesh(*s) for s in shapes]
+    rng = np.random.default_rng(4)
+    values = [rng.standard_normal((len(meshes), n)) * 1e-2 for _, n in updates]
+    table = np.zeros((len(meshes), STEPS))
+    for (t0, n), v in zip(updates, values):
+        table[:, t0:t0 + n] = v
+    table[:, :LEAD] = 0.0  # those steps were enqueued before the updates
+    with eng.Engine(meshes, "fp32") as a, eng.Engine(meshes, "fp32") as b:
+        a.set_wavelet(0, table, eng.ALL_MESHES)
+        a.step(STEPS)
+        want = _fields(a)
+        b.step(3)
+        b.reset()  # everything loaded, so that the updates overtake the steps where they can
+        b.step_async(LEAD)
+        for (t0, n), v in zip(updates, values):
+            b.set_wavelet(t0, v, eng.ALL_MESHES)
+        b.step(STEPS - LEAD)
+        got = _fields(b)
+    for x, y in zip(want, got):
+        assert np.array_equal(x, y)
+    assert np.abs(want[1]).max() > 0
