@@ -1790,6 +1790,14 @@ int dg_gpu_init(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const
   return init_context(out, meshes, n_meshes, opts, false);
 }
 
+// Whether the caller is capturing the context stream.
+static int capturing(dg_gpu_ctx* c, bool* yes) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(c->stream, &cap));
+  *yes = cap != cudaStreamCaptureStatusNone;
+  return DG_OK;
+}
+
 // Enqueue n steps on the context stream (graphs where they fit; the watchdog, when on,
 // synchronises at its checks).  The caller synchronises.
 static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
@@ -1798,9 +1806,8 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
   // a caller that captures the context stream gets plain launches: they take the step from the
   // device's counters, so the capture can be replayed, which the resident step's tags forbid, and
   // a graph cannot be launched into a capture
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(c->stream, &cap));
-  const bool plain = cap != cudaStreamCaptureStatusNone;
+  bool plain = false;
+  if (int rc = capturing(c, &plain)) return rc;
   long done = 0;
   while (done < n) {
     long chunk = n - done;
@@ -2564,6 +2571,10 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   for (int k = k0; k < k1; k++)
     if (t0 + n > c->mi[k].steps) return fail(DG_ERR_ARG, "wavelet window beyond a mesh's steps");
   CK(cudaSetDevice(c->device));
+  // an update goes into the table once, with this call's values: not to be replayed
+  bool captured = false;
+  if (int rc = capturing(c, &captured)) return rc;
+  if (captured) return fail(DG_ERR_STATE, "a wavelet update cannot be part of a capture");
   if (!c->subs.empty()) {
     for (int k = k0; k < k1; k++) {
       const int rc = dg_gpu_set_wavelet(c->subs[k].get(), 0, t0, n, w + (size_t)(k - k0) * n);

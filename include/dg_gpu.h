@@ -197,7 +197,7 @@ int dg_gpu_reset(dg_gpu_ctx *ctx);
  * past the steps enqueued so far) the copy does not wait for the steps in flight; up to 64
  * samples are staged and copied in stream order without any wait, and a longer update that an
  * earlier staged one may still overlap follows it there.  Of two updates of a sample the later
- * call's stays. */
+ * call's stays.  Refused (DG_ERR_STATE) while the caller captures the context's stream. */
 int dg_gpu_set_wavelet(dg_gpu_ctx *ctx, int mesh, long t0, long n, const double *w);
 
 /* ---- one mesh split over several contexts (one per GPU): domain decomposition --------------

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from conftest import pkg
+from stream_capture import Captured
 
 eng = pkg.engine
 pytestmark = pytest.mark.gpu
@@ -52,3 +53,25 @@ def test_the_last_update_of_a_sample_wins(updates, shapes, monkeypatch):
     for x, y in zip(want, got):
         assert np.array_equal(x, y)
     assert np.abs(want[1]).max() > 0
+
+
+@pytest.mark.parametrize("n", [1, 64, 65])
+def test_an_update_inside_a_capture_is_refused(n):
+    """An update goes into the wavelet table once, with the call's values: it cannot be part of a
+    capture, whatever its length."""
+    m = _mesh(9, 1)
+    with eng.Engine(m, "fp32") as e, eng.Engine(m, "fp32") as fresh:
+        e.set_wavelet(0, np.zeros(1))
+        with pytest.raises(eng.DGError):
+            with Captured(e) as g:
+                e.step_async(1)
+                e.set_wavelet(1, np.ones(n))
+        g.close()
+        e.reset()
+        for x in (e, fresh):  # the context works on
+            x.set_wavelet(0, np.full(70, 1e-3))
+            x.set_wavelet(3, np.full(n, 2e-3))
+            x.step(80)
+        for a, b in zip(_fields(e), _fields(fresh)):
+            assert np.array_equal(a, b)
+        assert np.abs(_fields(e)[1]).max() > 0
