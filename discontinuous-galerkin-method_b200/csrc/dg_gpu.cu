@@ -1031,6 +1031,11 @@ int launch_wave(dg_gpu_ctx* c) {
   if (!k) return fail(DG_ERR_UNSUPPORTED, "no wavefront step for this shot count");
   const dim3 bl(c->block), g(c->wave_persistent ? c->blocks_p : c->blocks_v);
   c->wave_ran = true;
+  // one block per ticket: the step comes out of the tickets, which resident steps leave behind
+  if (c->resident && !c->wave_persistent) {
+    k_wave_sync<<<1, 1, 0, c->stream>>>(c->d_ctr, c->wv.tickets, (unsigned)c->blocks_v);
+    CK(cudaGetLastError());
+  }
   k<<<g, bl, wave_smem(c), c->stream>>>(c->ops2, c->md_f[0], c->wv, c->d_ctr);
   return DG_OK;
 }
