@@ -154,6 +154,8 @@ struct dg_gpu_ctx {
   int res_blocks = 0, res_threads = 0;
   size_t res_smem = 0;
   unsigned res_seq = 1;
+  // the device's step counter may be ahead of t: the caller has captured steps and may replay them
+  bool count_on_device = false;
   Resident rs{};
   int* res_error = nullptr;
   // a batch of meshes stepped as one context per mesh, side by side: the contexts, the order in
@@ -1177,6 +1179,8 @@ int build_resident(dg_gpu_ctx* c) {
   if ((rc = c->alloc(&w.pt, mt * w.ps)) || (rc = c->alloc(&w.pv, mv * w.ps))) return rc;
   CK(cudaMemsetAsync(w.pt, 0, mt * w.ps * sizeof(uint4), c->stream));
   CK(cudaMemsetAsync(w.pv, 0, mv * w.ps * sizeof(uint4), c->stream));
+  if ((rc = c->alloc(&w.arrived, 1))) return rc;
+  CK(cudaMemsetAsync(w.arrived, 0, sizeof(unsigned), c->stream));
   CK(cudaHostAlloc(&c->res_error, sizeof(int), cudaHostAllocMapped));
   *c->res_error = 0;
   CK(cudaHostGetDevicePointer(&w.error, c->res_error, 0));
@@ -1193,11 +1197,11 @@ int build_resident(dg_gpu_ctx* c) {
 
 // nsteps steps in one launch (cooperative: blocks wait for one another's messages)
 int launch_resident(dg_gpu_ctx* c, int nsteps) {
-  long long t0 = c->t;
+  long long from = c->count_on_device ? -1 : c->t;
   unsigned seq = c->res_seq;
   void* ops = c->is_double ? (void*)&c->ops_d : (void*)&c->ops_f;  // FP32: operators are constants
   void* mesh = c->is_double ? (void*)&c->md_d[0] : (void*)&c->md_f[0];
-  void* args[] = {ops, mesh, &c->rs, &c->d_ctr, &t0, &nsteps, &seq};
+  void* args[] = {ops, mesh, &c->rs, &c->d_ctr, &from, &nsteps, &seq};
   c->res_seq += (unsigned)nsteps + 1u;
   CK(cudaLaunchCooperativeKernel(resident_kernel(c), dim3(c->res_blocks), dim3(c->res_threads), args, c->res_smem,
                                  c->stream));
@@ -1813,6 +1817,7 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
   // a graph cannot be launched into a capture
   bool plain = false;
   if (int rc = capturing(c, &plain)) return rc;
+  c->count_on_device = c->count_on_device || plain;
   long done = 0;
   while (done < n) {
     long chunk = n - done;
@@ -2365,6 +2370,7 @@ int dg_gpu_half_step(dg_gpu_ctx* c, int half) {
   if (half == 0 && c->t + 1 > c->max_steps) return fail(DG_ERR_STATE, "stepping past the end of the wavelet table");
   CK(cudaSetDevice(c->device));
   int rc = DG_OK;
+  c->count_on_device = true;  // they may be part of a capture
   if (c->subs.empty()) rc = launch_step(c, nullptr, nullptr, nullptr, half == 0 ? 1 : 2);
   for (auto& sub : c->subs) {
     if (half == 0 ? sub->t >= sub->max_steps : !sub->half_pending) continue;  // past its last step
@@ -2433,6 +2439,7 @@ int dg_gpu_half_step_part(dg_gpu_ctx* c, int half, int part) {
   }
   CK(cudaSetDevice(c->device));
   const bool closes = (c->part_done | part) == 3;
+  c->count_on_device = true;
   int rc = launch_part(c, half, part, closes && half == 1);
   if (rc) return rc;
   c->part_done |= part;

@@ -45,6 +45,7 @@ struct Resident {
   const int* rec_start;  // [blocks + 1] receivers of each block:
   const int* rec_list;   //   rec_list[rec_start[b] .. rec_start[b+1])
   int* error;
+  unsigned* arrived;     // blocks that have read the step counter (0 between launches)
   unsigned spin_limit;
 };
 
@@ -157,19 +158,28 @@ struct ArithRef {
 template <class A> constexpr bool is_ref = false;
 template <> constexpr bool is_ref<ArithRef> = true;
 
-// `nsteps` steps from step t0.  The stresses held between two steps carry the sponge factor of
+// `nsteps` steps from step `from`, or, if that is negative (the device's counter may be ahead of the host:
+// a caller replays captured steps), from the step the counter holds, as the other forms of the step
+// take it.  The counter costs a one-step call 0.5 us (its load, and the blocks counting themselves so
+// that the last to have read it advances it), so it is read only there.  The stresses held between two steps carry the sponge factor of
 // the coming step already (those in global memory do not), so neighbours read them as they are;
 // the stress tag of step s is seq + s, the velocity tag seq + s + 1.
 template <class A, bool KAHAN, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant__ typename A::Ops ops,
                                                            const __grid_constant__ MeshDev<typename A::R> m,
                                                            const __grid_constant__ Resident w,
-                                                           Counters* __restrict__ ctr, long long t0, int nsteps,
+                                                           Counters* __restrict__ ctr, long long from, int nsteps,
                                                            unsigned seq) {
   using V = typename A::V;
   using R = typename A::R;
   constexpr int SV = sizeof(V) / sizeof(R);  // shots of a lane
   constexpr bool REF = is_ref<A>;
+  long long t0 = from;
+  if (from < 0) {
+    t0 = *(volatile const long long*)&ctr->v;
+    nsteps = (int)min((long long)nsteps, m.steps - t0);
+    if (nsteps <= 0) return;
+  }
   extern __shared__ __align__(16) unsigned char res_smem[];
   V* const sV = reinterpret_cast<V*>(res_smem);  // [12][nls] Vx, Vz
   V* const sT = sV + 12 * w.nls;                 // [18][nls] Txx, Tzz, Txz, sponge factor applied
@@ -247,6 +257,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
           for (int f = 0; f < 3; f++) g[(f * NP + k) * nls] = v[3 * k + f];
       }
       __syncthreads();
+      if (from < 0 && s == 0 && l == 0 && atomicAdd(w.arrived, 1u) == gridDim.x - 1) {
+        *w.arrived = 0;
+        ctr->v = t0 + nsteps;
+        ctr->s = t0 + nsteps - 1;
+      }
       if (mine) {
         if constexpr (!REF) {
 #pragma unroll
@@ -396,7 +411,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
       for (int p = 0; p < 30; p++) *state_at<V>(m.C, m, e, p, q) = cc[p];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (from >= 0 && blockIdx.x == 0 && threadIdx.x == 0) {
     ctr->v = t0 + nsteps;
     ctr->s = t0 + nsteps - 1;
   }

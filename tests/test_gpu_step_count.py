@@ -68,3 +68,44 @@ def test_timed_steps_after_resident_ones(precision, how, tmp_path, monkeypatch):
     for a, b in zip(want, got):
         assert np.array_equal(a, b)
     assert np.abs(want[-1]).max() > 0
+
+
+# one mesh whose own steps stay on the SMs (one shot; 16, whose captured steps are wavefronts; 3), two
+# launches a step, a padded wavefront, a batch stepped mesh by mesh
+REPLAYS = [([(10, 1)], "fp32", {}), ([(10, 1)], "fp64", {}), ([(10, 16)], "fp32", {}), ([(12, 3)], "fp32_kahan", {}),
+           ([(10, 1)], "fp64", {"DG_RESIDENT": "0"}), ([(10, 24)], "fp32", {"DG_RESIDENT": "0", "DG_WAVE_MIN": "0"}),
+           ([(9, 1), (12, 4), (5, 2)], "fp32", {"DG_BATCH_BY_MESH": "1"})]
+
+
+@pytest.mark.parametrize("shapes,precision,env", REPLAYS)
+@pytest.mark.parametrize("n", [1, 7])
+def test_steps_after_replays(shapes, precision, env, n, monkeypatch):
+    """A capture of n steps replayed three times, then steps through the engine: they go on where the
+    replays ended (the host counts a captured call once)."""
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    meshes = [_mesh(*s) for s in shapes]
+    with eng.Engine(meshes, precision) as e:
+        _load(e)
+        e.step(2 + 3 * n + 20)
+        want = _fields(e)
+    with eng.Engine(meshes, precision) as e:
+        _load(e)
+        e.step(2)
+        with Captured(e) as g:
+            e.step_async(n)
+        g.launch(3)
+        e.step(20)
+        assert e.steps_done == 2 + n + 20
+        got = _fields(e)
+        g.close()
+        # what lies past the table by the device's count is skipped there, and a reset starts anew
+        e.step(STEPS - e.steps_done)
+        assert all(np.isfinite(a).all() for a in _fields(e))
+        e.reset()
+        _load(e)
+        e.step(2 + 3 * n + 20)
+        again = _fields(e)
+    for a, b, c in zip(want, got, again):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+    assert np.abs(want[0]).max() > 0
