@@ -156,6 +156,7 @@ struct dg_gpu_ctx {
   unsigned res_seq = 1;
   // the device's step counter may be ahead of t: the caller has captured steps and may replay them
   bool count_on_device = false;
+  bool in_capture = false;  // the steps enqueued last went into a caller's capture
   Resident rs{};
   int* res_error = nullptr;
   // a batch of meshes stepped as one context per mesh, side by side: the contexts, the order in
@@ -1817,6 +1818,7 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
   // a graph cannot be launched into a capture
   bool plain = false;
   if (int rc = capturing(c, &plain)) return rc;
+  c->in_capture = plain;
   c->count_on_device = c->count_on_device || plain;
   long done = 0;
   while (done < n) {
@@ -1888,13 +1890,14 @@ static int ensure_event(cudaEvent_t* ev) {
   return DG_OK;
 }
 
-// Records a step mark after the work enqueued so far.
+// Records a step mark after the work enqueued so far.  A mark inside a capture orders the captured work
+// only: no fetch may wait for it.
 static int mark_steps(dg_gpu_ctx* c) {
   auto& m = c->marks[c->mark_next];
   int rc = ensure_event(&m.ev);
   if (rc) return rc;
   CK(cudaEventRecord(m.ev, c->stream));
-  m.t_end = c->t;
+  m.t_end = c->in_capture ? -1 : c->t;
   c->mark_next = (c->mark_next + 1) % dg_gpu_ctx::kMarks;
   return DG_OK;
 }

@@ -109,3 +109,28 @@ def test_steps_after_replays(shapes, precision, env, n, monkeypatch):
     for a, b, c in zip(want, got, again):
         assert np.array_equal(a, b) and np.array_equal(a, c)
     assert np.abs(want[0]).max() > 0
+
+
+@pytest.mark.parametrize("shapes,precision,env", REPLAYS[:-1])
+def test_traces_after_replays(shapes, precision, env, monkeypatch):
+    """Traces of any window are to be had after a capture and its replays: of the captured call's
+    steps, of those before, and of those after it."""
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    meshes, n = [_mesh(*s) for s in shapes], 7
+    with eng.Engine(meshes, precision) as a, eng.Engine(meshes, precision) as e:
+        _load(a)
+        _load(e)
+        a.step(2 + n + 20)
+        e.step(2)
+        with Captured(e) as g:
+            e.step_async(n)
+        g.launch()
+        for t0, steps in ((2, n), (0, 2), (0, 2 + n)):
+            for x, y in zip(a.fetch_traces(t0, steps, eng.ALL_MESHES), e.fetch_traces(t0, steps, eng.ALL_MESHES)):
+                assert np.array_equal(x, y)
+        e.step(20)
+        for t0, steps in ((0, 2 + n), (2, n + 20), (0, 2 + n + 20)):
+            for x, y in zip(a.fetch_traces(t0, steps, eng.ALL_MESHES), e.fetch_traces(t0, steps, eng.ALL_MESHES)):
+                assert np.array_equal(x, y)
+        g.close()
