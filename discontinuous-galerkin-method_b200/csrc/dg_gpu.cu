@@ -154,8 +154,9 @@ struct dg_gpu_ctx {
   int res_blocks = 0, res_threads = 0;
   size_t res_smem = 0;
   unsigned res_seq = 1;
-  // the device's step counter may be ahead of t: the caller has captured steps and may replay them
-  bool count_on_device = false;
+  // the caller has captured steps, or may have, and may replay them: the device's step counter may be
+  // ahead of t, and a batch's meshes are changed by work on the context stream
+  bool may_replay = false;
   bool in_capture = false;  // the steps enqueued last went into a caller's capture
   Resident rs{};
   int* res_error = nullptr;
@@ -1198,7 +1199,7 @@ int build_resident(dg_gpu_ctx* c) {
 
 // nsteps steps in one launch (cooperative: blocks wait for one another's messages)
 int launch_resident(dg_gpu_ctx* c, int nsteps) {
-  long long from = c->count_on_device ? -1 : c->t;
+  long long from = c->may_replay ? -1 : c->t;
   unsigned seq = c->res_seq;
   void* ops = c->is_double ? (void*)&c->ops_d : (void*)&c->ops_f;  // FP32: operators are constants
   void* mesh = c->is_double ? (void*)&c->md_d[0] : (void*)&c->md_f[0];
@@ -1571,6 +1572,10 @@ static int sub_end(dg_gpu_ctx* c, dg_gpu_ctx* sub) {
   CK(cudaStreamWaitEvent(c->stream, c->ev_fork, 0));
   return DG_OK;
 }
+// The same around calls that the mesh's own stream orders, but for replayed captures: those run on the
+// context's stream alone.
+static int replays_begin(dg_gpu_ctx* c, dg_gpu_ctx* sub) { return c->may_replay ? sub_begin(c, sub) : DG_OK; }
+static int replays_end(dg_gpu_ctx* c, dg_gpu_ctx* sub) { return c->may_replay ? sub_end(c, sub) : DG_OK; }
 
 static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts_in,
                         bool member) {
@@ -1819,7 +1824,7 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
   bool plain = false;
   if (int rc = capturing(c, &plain)) return rc;
   c->in_capture = plain;
-  c->count_on_device = c->count_on_device || plain;
+  c->may_replay = c->may_replay || plain;
   long done = 0;
   while (done < n) {
     long chunk = n - done;
@@ -1957,6 +1962,7 @@ static int enqueue_subs(dg_gpu_ctx* c, long n) {
     CK(cudaStreamWaitEvent(sub->stream, last[at], 0));
     int rc = enqueue_steps(sub, m, false);
     if (rc || (rc = mark_steps(sub))) return rc;
+    c->may_replay = c->may_replay || sub->may_replay;
     const cudaEvent_t done = sub->marks[(sub->mark_next + dg_gpu_ctx::kMarks - 1) % dg_gpu_ctx::kMarks].ev;
     if (alone) {
       std::fill(last, last + kChains, done);
@@ -2173,8 +2179,8 @@ int dg_gpu_fetch_traces(dg_gpu_ctx* c, int mesh, long t0, long n, double* dst_x,
   CK(cudaSetDevice(c->device));
   long long at = 0;
   for (int k = k0; k < k1; k++) {
-    const int rc = fetch_traces_enqueue(c->subs[k].get(), 0, t0, n, dst_x + at, dst_z + at);
-    if (rc) return rc;
+    int rc = replays_begin(c, c->subs[k].get());
+    if (rc || (rc = fetch_traces_enqueue(c->subs[k].get(), 0, t0, n, dst_x + at, dst_z + at))) return rc;
     at += (long long)n * c->mi[k].n_rec * c->mi[k].S;
   }
   for (int k = k0; k < k1; k++) CK(cudaStreamSynchronize(c->subs[k]->copy_stream));
@@ -2244,6 +2250,7 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
   for (long j = 0; j < J; j++) {
     const int slot = (int)(j & 1);
     if ((rc = all == c ? enqueue_steps(c, every, false) : enqueue_subs(all, every))) return rc;
+    if (all != c && (rc = replays_begin(all, c))) return rc;
     // the device slot is free once the copy of snapshot j - 2 has finished
     if (j >= 2) CK(cudaStreamWaitEvent(c->stream, c->snap_copy[slot], 0));
     double* dslot = c->snap_dev + (size_t)slot * 2 * c->snap_elems;
@@ -2269,7 +2276,11 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
 
 int dg_gpu_fetch(dg_gpu_ctx* c, int what, int mesh, int shot, double* dst) {
   if (!c || !dst || mesh < 0 || mesh >= (int)c->mi.size()) return fail(DG_ERR_ARG, "bad arguments");
-  if (!c->subs.empty()) return dg_gpu_fetch(c->subs[mesh].get(), what, 0, shot, dst);
+  if (!c->subs.empty()) {
+    CK(cudaSetDevice(c->device));
+    const int rc = replays_begin(c, c->subs[mesh].get());
+    return rc ? rc : dg_gpu_fetch(c->subs[mesh].get(), what, 0, shot, dst);
+  }
   const MeshHostInfo& h = c->mi[mesh];
   const bool all = shot == DG_ALL_SHOTS && what >= DG_VX && what <= DG_TXZ;
   if (!all && (shot < 0 || shot >= h.S)) return fail(DG_ERR_ARG, "shot out of range");
@@ -2326,7 +2337,11 @@ int dg_gpu_fetch(dg_gpu_ctx* c, int what, int mesh, int shot, double* dst) {
 
 int dg_gpu_load(dg_gpu_ctx* c, int what, int mesh, int shot, const double* src) {
   if (!c || !src || mesh < 0 || mesh >= (int)c->mi.size()) return fail(DG_ERR_ARG, "bad arguments");
-  if (!c->subs.empty()) return dg_gpu_load(c->subs[mesh].get(), what, 0, shot, src);
+  if (!c->subs.empty()) {
+    CK(cudaSetDevice(c->device));
+    const int rc = replays_begin(c, c->subs[mesh].get());
+    return rc ? rc : dg_gpu_load(c->subs[mesh].get(), what, 0, shot, src);
+  }
   const MeshHostInfo& h = c->mi[mesh];
   if (shot < 0 || shot >= h.S) return fail(DG_ERR_ARG, "shot out of range");
   if (what < DG_VX || what > DG_TXZ) return fail(DG_ERR_STATE, "only fields can be loaded");
@@ -2373,7 +2388,7 @@ int dg_gpu_half_step(dg_gpu_ctx* c, int half) {
   if (half == 0 && c->t + 1 > c->max_steps) return fail(DG_ERR_STATE, "stepping past the end of the wavelet table");
   CK(cudaSetDevice(c->device));
   int rc = DG_OK;
-  c->count_on_device = true;  // they may be part of a capture
+  c->may_replay = true;  // they may be part of a capture
   if (c->subs.empty()) rc = launch_step(c, nullptr, nullptr, nullptr, half == 0 ? 1 : 2);
   for (auto& sub : c->subs) {
     if (half == 0 ? sub->t >= sub->max_steps : !sub->half_pending) continue;  // past its last step
@@ -2442,7 +2457,7 @@ int dg_gpu_half_step_part(dg_gpu_ctx* c, int half, int part) {
   }
   CK(cudaSetDevice(c->device));
   const bool closes = (c->part_done | part) == 3;
-  c->count_on_device = true;
+  c->may_replay = true;
   int rc = launch_part(c, half, part, closes && half == 1);
   if (rc) return rc;
   c->part_done |= part;
@@ -2512,6 +2527,7 @@ static int halo_copy(dg_gpu_ctx* c, int mesh, int what, void* buf, bool pack, bo
   if (!c->subs.empty()) {
     CK(cudaSetDevice(c->device));
     dg_gpu_ctx* sub = c->subs[mesh].get();
+    c->may_replay = true;  // may be part of a capture
     int rc = sub_begin(c, sub);
     if (rc || (rc = halo_copy(sub, 0, what, buf, pack, sync))) return rc;
     return sub_end(c, sub);
@@ -2592,8 +2608,9 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   if (captured) return fail(DG_ERR_STATE, "a wavelet update cannot be part of a capture");
   if (!c->subs.empty()) {
     for (int k = k0; k < k1; k++) {
-      const int rc = dg_gpu_set_wavelet(c->subs[k].get(), 0, t0, n, w + (size_t)(k - k0) * n);
-      if (rc) return rc;
+      dg_gpu_ctx* sub = c->subs[k].get();
+      int rc = replays_begin(c, sub);
+      if (rc || (rc = dg_gpu_set_wavelet(sub, 0, t0, n, w + (size_t)(k - k0) * n)) || (rc = replays_end(c, sub))) return rc;
     }
     return DG_OK;
   }

@@ -111,7 +111,7 @@ def test_steps_after_replays(shapes, precision, env, n, monkeypatch):
     assert np.abs(want[0]).max() > 0
 
 
-@pytest.mark.parametrize("shapes,precision,env", REPLAYS[:-1])
+@pytest.mark.parametrize("shapes,precision,env", REPLAYS)
 def test_traces_after_replays(shapes, precision, env, monkeypatch):
     """Traces of any window are to be had after a capture and its replays: of the captured call's
     steps, of those before, and of those after it."""
