@@ -2644,9 +2644,10 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   }
   // samples that no enqueued step reads (t0 at or past the steps enqueued so far) go over the
   // copy stream, and the context stream waits for them, so steps in flight keep running;
-  // otherwise, and where a staged copy of an earlier call could still land on them, the copy
-  // follows the enqueued work on the context stream
-  const bool ahead = t0 >= c->t && t0 >= c->staged_end;
+  // otherwise, and where a staged copy of an earlier call could still land on them or replayed
+  // steps that the host has not counted may read them, the copy follows the enqueued work on the
+  // context stream
+  const bool ahead = t0 >= c->t && t0 >= c->staged_end && !c->may_replay;
   int rc;
   if (ahead && ((rc = ensure_copy_stream(c)) || (rc = ensure_event(&c->ev_wavelet)))) return rc;
   cudaStream_t st = ahead ? c->copy_stream : c->stream;

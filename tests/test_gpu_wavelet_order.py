@@ -75,3 +75,30 @@ def test_an_update_inside_a_capture_is_refused(n):
         for a, b in zip(_fields(e), _fields(fresh)):
             assert np.array_equal(a, b)
         assert np.abs(_fields(e)[1]).max() > 0
+
+
+@pytest.mark.parametrize("n", [40, 200])
+@pytest.mark.parametrize("shapes", [((50, 1),), ((20, 4), (50, 1))])
+def test_replayed_steps_in_flight_read_the_samples_of_before(n, shapes, monkeypatch):
+    """A capture of 500 steps replayed three times reads 1,500 samples, of which the host has counted
+    500: an update past those does not overtake the replays."""
+    monkeypatch.setenv("DG_BATCH_BY_MESH", "1")
+    meshes = [_mesh(*s) for s in shapes]
+    table = np.random.default_rng(5).standard_normal((len(meshes), STEPS)) * 1e-3
+    with eng.Engine(meshes, "fp32") as a, eng.Engine(meshes, "fp32") as b:
+        for e in (a, b):
+            e.set_wavelet(0, table, eng.ALL_MESHES)
+        a.step(1500)
+        with Captured(b) as g:
+            b.step_async(500)
+        g.launch()
+        b.synchronize()
+        b.reset()
+        b.step(500)
+        g.launch(2)
+        b.set_wavelet(700, np.full((len(meshes), n), 0.5), eng.ALL_MESHES)
+        got = _fields(b)
+        g.close()
+        for x, y in zip(_fields(a), got):
+            assert np.array_equal(x, y)
+        assert np.abs(got[1]).max() > 0
