@@ -1382,6 +1382,7 @@ int zero_state(dg_gpu_ctx* c) {
     CK(cudaMemsetAsync(c->wv.error, 0, sizeof(int), c->stream));
   }
   CK(cudaStreamSynchronize(c->stream));
+  if (c->res_error) *c->res_error = 0;  // in host memory: once no launch can set it any more
   c->t = 0;
   c->staged_end = 0;
   for (auto& m : c->marks) m.t_end = -1;  // no step mark covers the new run's steps
