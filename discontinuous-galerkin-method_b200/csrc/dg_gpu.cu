@@ -1845,7 +1845,7 @@ static int enqueue_steps(dg_gpu_ctx* c, long n, bool timed) {
         c->stats.ms_stress += b;
       }
       c->stats.launches += (c->wave || c->mx_persistent ? 1 : 2) * chunk;
-    } else if (c->resident && !plain) {
+    } else if (c->resident && !plain && c->stall_unit < 0) {  // a stalled wavefront unit is to be waited for
       chunk = std::min<long>(chunk, 1L << 16);
       int rc = launch_resident(c, (int)chunk);
       if (rc) return rc;

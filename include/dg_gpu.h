@@ -287,7 +287,8 @@ int dg_gpu_flush_l2(dg_gpu_ctx *ctx);
 /* Test hook of the wavefront step (no counterpart in the reference): unit >= 0 makes the stress
  * update of that warp unit wait on a flag no warp ever publishes, so its wait reaches its limit
  * (about a second) and the next dg_gpu_step returns DG_ERR_TIMEOUT, the state of that step being
- * wrong; unit < 0 undoes it.  dg_gpu_reset then gives a context that steps as a fresh one.  On a
+ * wrong; unit < 0 undoes it.  dg_gpu_reset then gives a context that steps as a fresh one.  A small
+ * mesh that has a wavefront form beside its resident one steps in the wavefront form meanwhile.  On a
  * persistent batch of meshes (kernel family 8) unit >= 0 makes its grid barrier wait for one
  * block more than the grid holds, with a short limit (milliseconds), to the same effect.
  * DG_ERR_UNSUPPORTED when the context has neither (a batch that steps mesh by mesh waits nowhere). */

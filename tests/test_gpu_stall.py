@@ -40,3 +40,23 @@ def test_reset_forgets_an_unreported_timeout(monkeypatch):
         e.reset()
         e.synchronize()
         _timeout(e.step, 3)  # the hook still holds one message back
+
+
+def test_the_wavefront_hook_on_a_context_that_steps_resident():
+    """16 shots on a small mesh have a wavefront form beside the resident one: with a unit of it
+    stalled, every step call reports the timeout, and with the hook taken back and a reset the
+    context steps as a fresh one."""
+    m = _mesh(10, 16)
+    with eng.Engine(m, "fp32") as e:
+        want = _run(e)
+    with eng.Engine(m, "fp32") as e:
+        e.step(2)
+        e.debug_stall_wave(3)
+        _timeout(e.step, 3)
+        _timeout(e.step_timed, 1)
+        e.debug_stall_wave(-1)
+        e.reset()
+        got = _run(e)
+        assert e.stats()["launches"] == 1
+    for a, b in zip(want, got):
+        assert np.array_equal(a, b)
