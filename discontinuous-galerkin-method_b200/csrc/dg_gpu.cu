@@ -160,6 +160,7 @@ struct dg_gpu_ctx {
   bool in_capture = false;  // the steps enqueued last went into a caller's capture
   Resident rs{};
   int* res_error = nullptr;
+  int res_stalled = -1, res_stall_saved = 0;  // element whose message DG_RESIDENT_STALL holds back, its slot
   // a batch of meshes stepped as one context per mesh, side by side: the contexts, the order in
   // which a step call takes them (costliest first), the fork event of a call
   std::vector<std::unique_ptr<dg_gpu_ctx>> subs;
@@ -1062,6 +1063,7 @@ int resident_lanes(const dg_gpu_ctx* c, bool is_double, bool one, bool kahan) {
   if (is_double) return kernel_resident_d(false).max_threads;
   return one ? kernel_resident_f1(kahan, false).max_threads : kernel_resident_f2(kahan, false).max_threads;
 }
+constexpr unsigned kResidentSpins = 1u << 20;  // poll limit: a million polls of an L2 line, about a second
 bool resident_off() {
   const char* env = getenv("DG_RESIDENT");
   return env && atoi(env) == 0;
@@ -1151,7 +1153,7 @@ int build_resident(dg_gpu_ctx* c) {
   w.nls = w.nl + (int)(most * H) + 1;
   w.H = H;
   w.ps = std::max<long long>(1, (long long)slots * H);
-  w.spin_limit = 1u << 20;  // a million polls of an L2 line: about a second
+  w.spin_limit = kResidentSpins;
   c->res_smem = 30 * vsize * w.nls;
   if (c->res_smem > (size_t)smem_max || 6L * w.nls > 65535) return DG_OK;
   c->res_blocks = nb;
@@ -1167,6 +1169,8 @@ int build_resident(dg_gpu_ctx* c) {
   if (getenv("DG_RESIDENT_STALL") && slots > 0) {
     for (long e = 0; e < K && w.spin_limit > 4096; e++)
       if (out[e].x >= 0) {
+        c->res_stalled = (int)e;
+        c->res_stall_saved = out[e].x;
         out[e].x = slots;
         w.spin_limit = 4096;
       }
@@ -1194,6 +1198,16 @@ int build_resident(dg_gpu_ctx* c) {
   w.rec_list = d_rl;
   c->resident = true;
   CK(cudaStreamSynchronize(c->stream));
+  return DG_OK;
+}
+
+// Takes DG_RESIDENT_STALL back.
+int resident_unstall(dg_gpu_ctx* c) {
+  int4* out = const_cast<int4*>(c->rs.out) + c->res_stalled;
+  CK(cudaMemcpyAsync(&out->x, &c->res_stall_saved, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  c->rs.spin_limit = kResidentSpins;
+  c->res_stalled = -1;
   return DG_OK;
 }
 
@@ -2574,6 +2588,10 @@ int dg_gpu_debug_stall_wave(dg_gpu_ctx* c, int unit) {
     c->mx_extra = unit >= 0 ? 1u : 0u;
     c->mx_spin = unit >= 0 ? (1u << 14) : (1u << 22);
     return DG_OK;
+  }
+  if (unit < 0 && c->res_stalled >= 0) {
+    CK(cudaSetDevice(c->device));
+    return resident_unstall(c);
   }
   if (!c->wave || c->wave_mid) return fail(DG_ERR_UNSUPPORTED, "this context has no wavefront step");
   if (unit >= c->wv.NU) return fail(DG_ERR_ARG, "unit out of range");

@@ -290,7 +290,9 @@ int dg_gpu_flush_l2(dg_gpu_ctx *ctx);
  * wrong; unit < 0 undoes it.  dg_gpu_reset then gives a context that steps as a fresh one.  A small
  * mesh that has a wavefront form beside its resident one steps in the wavefront form meanwhile.  On a
  * persistent batch of meshes (kernel family 8) unit >= 0 makes its grid barrier wait for one
- * block more than the grid holds, with a short limit (milliseconds), to the same effect.
+ * block more than the grid holds, with a short limit (milliseconds), to the same effect.  A context
+ * made with DG_RESIDENT_STALL in the environment holds back one message of its resident step (short
+ * limit, too); unit < 0 undoes that.
  * DG_ERR_UNSUPPORTED when the context has neither (a batch that steps mesh by mesh waits nowhere). */
 int dg_gpu_debug_stall_wave(dg_gpu_ctx *ctx, int unit);
 

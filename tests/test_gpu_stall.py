@@ -60,3 +60,21 @@ def test_the_wavefront_hook_on_a_context_that_steps_resident():
         assert e.stats()["launches"] == 1
     for a, b in zip(want, got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_a_resident_context_recovers(precision, monkeypatch):
+    """After a timeout of the resident step, the hook taken back and a reset, the context steps as a
+    fresh one."""
+    m = _mesh(20, 1)
+    with eng.Engine(m, precision) as e:
+        want = _run(e)
+    monkeypatch.setenv("DG_RESIDENT_STALL", "1")
+    with eng.Engine(m, precision) as e:
+        _timeout(e.step, 3)
+        e.debug_stall_wave(-1)
+        e.reset()
+        got = _run(e)
+        assert e.stats()["launches"] == 1
+    for a, b in zip(want, got):
+        assert np.array_equal(a, b)
