@@ -134,7 +134,7 @@ struct dg_gpu_ctx {
   // x2 is then the stored shots, for the resident step), and for half steps of a wave_mid context
   bool gen_p2 = false;
   bool form_auto = true;  // the step's form is left to the engine (dg_gpu_opts::wavefront = 0)
-  bool wave_ran = false;  // wavefront launches since the error word was last read
+  bool wave_ran = false;  // wavefront launches since the error word was last read, or captured ones
   bool no_halves = false; // no half steps, as for a wavefront context (an automatic one that chose two launches)
   bool wave_mid = false;  // a wavefront context of a shot count between the powers of two
   bool wave = false;  // one launch per step (k_step_wave / k_step_wave_p), RCM order, schedule in wv
@@ -1365,7 +1365,7 @@ int check_wave(dg_gpu_ctx* c) {
     return fail(DG_ERR_TIMEOUT, "a wait between blocks of the resident step reached its limit");
   }
   if (!c->wave || (c->resident && !c->wave_ran)) return DG_OK;
-  c->wave_ran = false;
+  c->wave_ran = c->may_replay;  // captured launches run again without the host
   int err = 0;
   CK(cudaMemcpyAsync(&err, c->wv.error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

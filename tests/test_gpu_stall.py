@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from conftest import pkg
+from stream_capture import Captured
 
 eng = pkg.engine
 pytestmark = pytest.mark.gpu
@@ -78,3 +79,24 @@ def test_a_resident_context_recovers(precision, monkeypatch):
         assert e.stats()["launches"] == 1
     for a, b in zip(want, got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("resident", ["0", "1"])
+def test_a_timeout_in_a_replayed_capture_is_reported(resident, monkeypatch):
+    """A captured wavefront step that stalls when it is replayed, after the captured call's own
+    report was asked for."""
+    monkeypatch.setenv("DG_RESIDENT", resident)
+    monkeypatch.setenv("DG_WAVE_MIN", "0")
+    with eng.Engine(_mesh(10, 16), "fp32") as e:
+        with Captured(e) as g:
+            e.step_async(2)
+        g.launch()
+        e.synchronize()
+        e.debug_stall_wave(3)
+        for _ in range(2):
+            g.launch()
+            _timeout(e.synchronize)
+        e.debug_stall_wave(-1)
+        g.launch()
+        e.synchronize()
+        g.close()
