@@ -36,6 +36,7 @@ int cuda_fail(cudaError_t e, const char* what, int line) {
   char buf[512];
   snprintf(buf, sizeof buf, "%s (line %d): %s", what, line, cudaGetErrorString(e));
   g_last = buf;
+  cudaGetLastError();  // reported here: the check behind the next launch is not to find it again
   return e == cudaErrorMemoryAllocation ? DG_ERR_NOMEM : DG_ERR_CUDA;
 }
 #define CK(x)                                                \
@@ -2241,7 +2242,7 @@ int dg_gpu_step_snapshots(dg_gpu_ctx* c, long n, long every, int mesh, int shot,
     int rc = c->alloc(&c->snap_dev, 4 * per);
     if (rc) return rc;
     void* hp = nullptr;
-    if (cudaMallocHost(&hp, 4 * per * sizeof(double)) != cudaSuccess) return fail(DG_ERR_NOMEM, "pinned snapshot ring");
+    CK(cudaMallocHost(&hp, 4 * per * sizeof(double)));
     c->snap_host = (double*)hp;
     c->snap_elems = per;
   }
@@ -2640,8 +2641,7 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   if (few > 0 && few <= 64) {
     if (!c->wave_host) {
       void* p = nullptr;
-      if (cudaMallocHost(&p, 2 * dg_gpu_ctx::kWave * sizeof(double)) != cudaSuccess)
-        return fail(DG_ERR_NOMEM, "pinned wavelet staging");
+      CK(cudaMallocHost(&p, 2 * dg_gpu_ctx::kWave * sizeof(double)));
       c->wave_host = (double*)p;
       for (auto& e : c->ev_wave) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
