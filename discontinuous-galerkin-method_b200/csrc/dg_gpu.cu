@@ -1668,7 +1668,12 @@ static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshe
       const long long K = meshes[k].K, lanes = resident_lanes(c.get(), false, false, c->kahan) / (even / 2);
       size_t free_b = 0, total_b = 0;
       CK(cudaMemGetInfo(&free_b, &total_b));
-      auto room = [&](int S) { return 30.0 * K * S * 4 * (c->kahan ? 2 : 1) < 0.8 * free_b; };
+      // padding shots only where the state, the trace table and the staging buffer leave a fifth free
+      const double rec = (double)std::max(1, meshes[k].n_rec), rows = (double)std::max(0L, meshes[k].n_steps);
+      auto room = [&](int S) {
+        const double state = 30.0 * K * S * 4 * (c->kahan ? 2 : 1), trace = 2.0 * rows * rec * S * 4;
+        return state + trace + 8.0 * (6.0 * K + rows * rec) < 0.8 * free_b;
+      };
       const bool small = lanes * c->num_sms >= K && !resident_off();
       if (!small && o.wavefront == 0 && Sw && K * meshes[k].n_shots >= wave_min(c->kahan, false) && room(Sw) &&
           K * (Sw / 2) < (1LL << 31)) {

@@ -61,3 +61,21 @@ def test_a_failed_context_leaves_nothing_for_the_next(monkeypatch):
             assert e.stats()["kernel_family"] == family
             e.step(8)
             assert all(np.isfinite(e.fetch(f)).all() for f in FIELDS)
+
+
+@pytest.mark.parametrize("env", [{}, {"DG_RESIDENT": "0"}, {"DG_RESIDENT": "0", "DG_WAVE_MIN": "0"}])
+def test_padded_shots_count_the_trace_table(env, monkeypatch):
+    """17 shots whose traces fill what is left but for half a shot's: there is no room for a padding
+    shot, so the counts' own kernels run unpadded."""
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    steps, receivers = 4000, 40000
+    m = _mesh(6, 17, steps)
+    m["receiver"] = np.tile(m["receiver"], (receivers // len(m["receiver"]) + 1, 1))[:receivers]
+    shot = steps * 2 * receivers * 4  # bytes of one shot's traces
+    with eng.Engine(_mesh(6, 17, 8), "fp32") as e:
+        e.step(8)
+    with Filled(17 * shot + steps * receivers * 8 + shot // 2):
+        with eng.Engine(m, "fp32") as e:
+            e.step(8)
+            assert e.steps_done == 8 and np.isfinite(e.fetch("Vz", 0, 16)).all()
