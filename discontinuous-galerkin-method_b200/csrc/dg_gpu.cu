@@ -1070,6 +1070,11 @@ bool resident_off() {
   return env && atoi(env) == 0;
 }
 
+int alloc_error_word(dg_gpu_ctx* c) {
+  CK(cudaHostAlloc(&c->res_error, sizeof(int), cudaHostAllocMapped));
+  return DG_OK;
+}
+
 // The resident step's tables, where a thread for every lane fits on the SMs at once (FP64 and two
 // shots a lane: 56,832 lanes, FP32 one shot 75,776, Kahan and the reference operators 37,888, Kahan one
 // shot 56,832): elements cut into runs
@@ -1177,18 +1182,24 @@ int build_resident(dg_gpu_ctx* c) {
       }
     w.ps += H;
   }
-  int *d_start, *d_slots, *d_rs, *d_rl, rc;
+  // what does not fit leaves the two launches a step: nothing of it is kept then
+  int *d_start, *d_slots, *d_rs, *d_rl;
   int4 *d_link, *d_out;
-  if ((rc = c->upload(&d_start, start)) || (rc = c->upload(&d_slots, sstart)) || (rc = c->upload(&d_link, link)) ||
-      (rc = c->upload(&d_out, out)) || (rc = c->upload(&d_rs, rstart)) || (rc = c->upload(&d_rl, rlist)))
-    return rc;
   const size_t mt = 3 * vsize / 4, mv = 2 * vsize / 4;  // messages of a face and lane
-  if ((rc = c->alloc(&w.pt, mt * w.ps)) || (rc = c->alloc(&w.pv, mv * w.ps))) return rc;
+  const size_t held = c->allocs.size();
+  int rc;
+  if ((rc = c->upload(&d_start, start)) || (rc = c->upload(&d_slots, sstart)) || (rc = c->upload(&d_link, link)) ||
+      (rc = c->upload(&d_out, out)) || (rc = c->upload(&d_rs, rstart)) || (rc = c->upload(&d_rl, rlist)) ||
+      (rc = c->alloc(&w.pt, mt * w.ps)) || (rc = c->alloc(&w.pv, mv * w.ps)) || (rc = c->alloc(&w.arrived, 1)) ||
+      (rc = alloc_error_word(c))) {
+    while (c->allocs.size() > held) c->release(c->allocs.back());
+    c->rs = Resident{};
+    c->res_stalled = -1;
+    return rc == DG_ERR_NOMEM ? DG_OK : rc;
+  }
   CK(cudaMemsetAsync(w.pt, 0, mt * w.ps * sizeof(uint4), c->stream));
   CK(cudaMemsetAsync(w.pv, 0, mv * w.ps * sizeof(uint4), c->stream));
-  if ((rc = c->alloc(&w.arrived, 1))) return rc;
   CK(cudaMemsetAsync(w.arrived, 0, sizeof(unsigned), c->stream));
-  CK(cudaHostAlloc(&c->res_error, sizeof(int), cudaHostAllocMapped));
   *c->res_error = 0;
   CK(cudaHostGetDevicePointer(&w.error, c->res_error, 0));
   w.e_start = d_start;

@@ -79,3 +79,40 @@ def test_padded_shots_count_the_trace_table(env, monkeypatch):
         with eng.Engine(m, "fp32") as e:
             e.step(8)
             assert e.steps_done == 8 and np.isfinite(e.fetch("Vz", 0, 16)).all()
+
+
+def test_no_room_for_the_resident_steps_messages(monkeypatch):
+    """The least memory in which a mesh steps in two launches, and a little more of it: the same mesh
+    is made and steps there too where the engine would keep it on the SMs."""
+    m = _mesh(150, 1, 12)
+
+    def run():
+        with eng.Engine(m, "fp64", reorder=False, graph_steps=-1) as e:
+            e.step(12)
+            return e.stats()["launches"], [e.fetch(f) for f in FIELDS]
+
+    launches, want = run()  # loads the kernels, too
+    assert launches == 1
+    monkeypatch.setenv("DG_RESIDENT", "0")
+    assert run()[0] == 24
+
+    def fits(leave):
+        with Filled(leave):
+            try:
+                run()
+                return True
+            except eng.DGError as err:
+                assert err.code == -3
+                return False
+
+    low, high = 0, 256  # in 2 MB
+    assert fits(high * 2 * MB)
+    while high - low > 1:
+        mid = (low + high) // 2
+        low, high = (low, mid) if fits(mid * 2 * MB) else (mid, high)
+    monkeypatch.setenv("DG_RESIDENT", "1")
+    for more in range(0, 9):
+        with Filled((high + more) * 2 * MB):
+            launches, got = run()
+        for a, b in zip(want, got):
+            assert np.array_equal(a, b)
