@@ -1541,6 +1541,8 @@ static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshe
 // meshes FP32 388 -> 352 and 419 -> 398, Kahan 724 -> 567 and 750 -> 611, FP64 772 -> 729 and
 // 785 -> 775; 24 of 80,000 lanes 274 -> 184 and 301 -> 268; 8 of 57,600 68 -> 43 and 81 -> 78; below
 // the line 8 of 14,400 19 -> 22 and 31 -> 66, 12 of 20,000 FP64 42 -> 42 and 54 -> 94.
+constexpr double kBatchLanes = 50000;
+static double batch_lanes(int precision, long K, int S) { return (double)K * S / (precision <= DG_FP64 ? 1 : 2); }
 static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
   const char* env = getenv("DG_BATCH_BY_MESH");
   if (n < 2 || o.variant != 0 || o.wavefront == 1 || o.autotune || o.block_threads || o.watchdog_every > 0 ||
@@ -1549,13 +1551,12 @@ static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
   double lanes = 0;
   for (int k = 0; k < n; k++) {
     if (!m[k].Vr || !m[k].Vs || !m[k].inverV || !m[k].S || m[k].K <= 0 || m[k].n_shots < 1) return false;
-    const double s = m[k].n_shots;
-    lanes += m[k].K * (o.precision <= DG_FP64 ? s : s / 2);
+    lanes += batch_lanes(o.precision, m[k].K, m[k].n_shots);
     if (k && (memcmp(m[k].Vr, m[0].Vr, 36 * sizeof(double)) || memcmp(m[k].Vs, m[0].Vs, 36 * sizeof(double)) ||
               memcmp(m[k].inverV, m[0].inverV, 36 * sizeof(double)) || memcmp(m[k].S, m[0].S, 54 * sizeof(double))))
       return false;
   }
-  return env ? true : lanes >= 50000.0 * n;
+  return env ? true : lanes >= kBatchLanes * n;
 }
 
 static int init_subs(dg_gpu_ctx* c, const dg_gpu_mesh* meshes, int n, const dg_gpu_opts& o) {
@@ -1963,14 +1964,18 @@ static int steps_done_event(dg_gpu_ctx* c, long t, cudaEvent_t* out) {
 // and of one: one chain 384 and 510, two 373 and 480, two after the large mesh 353 and 435, four
 // after it 353 and 405).
 static int enqueue_subs(dg_gpu_ctx* c, long n) {
-  constexpr int kChains = 4;
+  constexpr int kChains = 4, kSmallChains = 8;
   constexpr double kAlone = 150e6;  // bytes of state
   const auto bytes = [&](int k) {
     return 30.0 * (c->is_double ? 8 : 4) * (c->kahan ? 2 : 1) * c->subs[k]->mi[0].K * c->subs[k]->mi[0].S_pad;
   };
   // in a call of many steps no more chains than keep their states in L2 together (4 meshes of
   // 28,800 elements, 8 shots, 28 MB each: two chains 43.1 us a step, four 62.2); in a short one
-  // the gaps between launches cost more (24 meshes of 20,000, 8 shots, 5 steps a call: 265, 231)
+  // the gaps between launches cost more (24 meshes of 20,000, 8 shots, 5 steps a call: 265, 231).
+  // There a mesh below kBatchLanes takes about 15 us of its chain whatever its size, so those have
+  // chains of their own (calls of one: 6 uneven meshes of 3,000 to 188,000 lanes FP32 106 -> 80, FP64
+  // 169 -> 142; all meshes in one launch 91 and 148; twelve chains for all meshes cost 24 of 80,000
+  // lanes 297 instead of 268)
   int chains = kChains;
   if (n >= 16) {
     double held = 0;
@@ -1980,24 +1985,26 @@ static int enqueue_subs(dg_gpu_ctx* c, long n) {
     chains = std::max(chains, 2);
   }
   CK(cudaEventRecord(c->ev_fork, c->stream));
-  cudaEvent_t last[kChains];
-  double load[kChains] = {};
-  std::fill(last, last + kChains, c->ev_fork);
+  constexpr int kAll = kChains + kSmallChains;
+  cudaEvent_t last[kAll];
+  double load[kAll] = {};
+  std::fill(last, last + kAll, c->ev_fork);
   c->stats.launches = 0;
   for (int k : c->sub_order) {  // costliest first
     dg_gpu_ctx* sub = c->subs[k].get();
     const long m = std::min(n, sub->max_steps - sub->t);
     if (m <= 0) continue;  // past its last step
-    const double lanes = (double)sub->mi[0].K * sub->mi[0].S_pad;
-    const bool alone = bytes(k) > kAlone;
-    const int at = (int)(std::min_element(load, load + chains) - load);
+    const double lanes = batch_lanes(c->precision, sub->mi[0].K, sub->mi[0].S_pad);
+    const bool alone = bytes(k) > kAlone, own = n < 16 && lanes < kBatchLanes;
+    const int first = own ? kChains : 0, past = own ? kAll : chains;
+    const int at = (int)(std::min_element(load + first, load + past) - load);
     CK(cudaStreamWaitEvent(sub->stream, last[at], 0));
     int rc = enqueue_steps(sub, m, false);
     if (rc || (rc = mark_steps(sub))) return rc;
     c->may_replay = c->may_replay || sub->may_replay;
     const cudaEvent_t done = sub->marks[(sub->mark_next + dg_gpu_ctx::kMarks - 1) % dg_gpu_ctx::kMarks].ev;
     if (alone) {
-      std::fill(last, last + kChains, done);
+      std::fill(last, last + kAll, done);
     } else {
       last[at] = done;
       load[at] += lanes * m;
