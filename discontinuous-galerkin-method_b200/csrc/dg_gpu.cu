@@ -1533,14 +1533,19 @@ const char* dg_gpu_last_error(void) { return g_last.c_str(); }
 static int init_context(dg_gpu_ctx** out, const dg_gpu_mesh* meshes, int n_meshes, const dg_gpu_opts* opts, bool member);
 
 // Whether a batch is stepped mesh by mesh: the engine's own choice of kernels throughout, the
-// same operators for every mesh, no watchdog (it stops all meshes at the same step), and meshes of
-// 50,000 lanes on average, so that a mesh's launches keep the GPU busy while the host enqueues the
-// next (DG_BATCH_BY_MESH=0/1 overrides the size).  Each mesh then has the kernels of its own shot
-// count, its state in L2 for the whole call where it fits, and no mesh waits for the others' half
-// steps.  us a step against all meshes in each launch, calls of 50 steps and of one: 12 uneven
-// meshes FP32 388 -> 352 and 419 -> 398, Kahan 724 -> 567 and 750 -> 611, FP64 772 -> 729 and
-// 785 -> 775; 24 of 80,000 lanes 274 -> 184 and 301 -> 268; 8 of 57,600 68 -> 43 and 81 -> 78; below
-// the line 8 of 14,400 19 -> 22 and 31 -> 66, 12 of 20,000 FP64 42 -> 42 and 54 -> 94.
+// same operators for every mesh, no watchdog (it stops all meshes at the same step), and enough work.
+// Each mesh then has the kernels of its own shot count, its state in L2 for the whole call where it
+// fits, and no mesh waits for the others' half steps; but each has launches of its own.  In a one-step
+// call they cost about 8 us of host time a mesh, which 55,000 lanes a mesh outweigh; a mesh beyond
+// 90,000 lanes saves no more than one of 90,000, while a small one takes its few us a step, so those
+// must leave 50,000 on average (DG_BATCH_BY_MESH=0/1 overrides the size).
+// us a step, all meshes in each launch -> mesh by mesh, in calls of 50 steps and of one: 12 uneven
+// meshes FP32 388 -> 352 and 423 -> 395, Kahan 724 -> 567 and 750 -> 611, FP64 776 -> 731 and
+// 825 -> 804; 24 of 80,000 lanes 278 -> 184 and 305 -> 267; 8 of 57,600 71 -> 47 and 84 -> 79; 3 of 600,000
+// and 2 of 1,000 260 -> 251 and 286 -> 258.  Below the lines: 4 of 50,200 27 -> 20 and 39 -> 41; 8 of 14,400
+// 19 -> 22 and 32 -> 62; 12 of 20,000 FP64 42 -> 42 and 53 -> 84; 1 of 1.28 M and 23 of 1,000 194 -> 229 and
+// 220 -> 247; 1 of 600,000 and 11 of 1,000 99 -> 163 and 112 -> 148; 8 of 100,000 and 8 of 1,000 129 -> 139
+// and 143 -> 158.
 constexpr double kBatchLanes = 50000;
 static double batch_lanes(int precision, long K, int S) { return (double)K * S / (precision <= DG_FP64 ? 1 : 2); }
 static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
@@ -1548,15 +1553,17 @@ static bool batch_by_mesh(const dg_gpu_mesh* m, int n, const dg_gpu_opts& o) {
   if (n < 2 || o.variant != 0 || o.wavefront == 1 || o.autotune || o.block_threads || o.watchdog_every > 0 ||
       getenv("DG_MX_PERSISTENT") || (env && atoi(env) == 0))
     return false;
-  double lanes = 0;
+  double lanes = 0, counted = 0;
   for (int k = 0; k < n; k++) {
     if (!m[k].Vr || !m[k].Vs || !m[k].inverV || !m[k].S || m[k].K <= 0 || m[k].n_shots < 1) return false;
-    lanes += batch_lanes(o.precision, m[k].K, m[k].n_shots);
+    const double l = batch_lanes(o.precision, m[k].K, m[k].n_shots);
+    lanes += l;
+    counted += std::min(l, 90000.0);
     if (k && (memcmp(m[k].Vr, m[0].Vr, 36 * sizeof(double)) || memcmp(m[k].Vs, m[0].Vs, 36 * sizeof(double)) ||
               memcmp(m[k].inverV, m[0].inverV, 36 * sizeof(double)) || memcmp(m[k].S, m[0].S, 54 * sizeof(double))))
       return false;
   }
-  return env ? true : lanes >= kBatchLanes * n;
+  return env ? true : lanes >= 55000.0 * n && counted >= kBatchLanes * n;
 }
 
 static int init_subs(dg_gpu_ctx* c, const dg_gpu_mesh* meshes, int n, const dg_gpu_opts& o) {

@@ -127,9 +127,10 @@ typedef struct {
 	                            the bodies of 4 with a grid barrier between the halves (default for
 	                            batches of at least 16 work blocks per resident block),
 	                          9 batch of meshes, each stepped by a context of its own with the kernels of
-	                            a single mesh, several meshes side by side (default for batches of 50,000
-	                            lanes a mesh on average, a lane being one element and shot in FP64, one
-	                            and two shots in FP32).
+	                            a single mesh, several meshes side by side (default for batches of 55,000
+	                            lanes a mesh on average, 50,000 with no mesh counted for more than
+	                            90,000, a lane being one element and shot in FP64, one element and two
+	                            shots in FP32).
 	                          A single mesh whose state fits in the SMs' registers runs dg_gpu_step in one
 	                          cooperative launch for all its steps; the family reported is then that of
 	                          its other calls (half steps, timed and profiled steps), with the same bits */

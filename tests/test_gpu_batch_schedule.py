@@ -39,3 +39,17 @@ def test_calls_of_any_length(precision, monkeypatch):
     for a, b in zip(*out):
         assert np.array_equal(a, b)
     assert np.abs(out[0][0]).max() > 0
+
+
+# (cells per side, shots) of the meshes: like sizes on both sides of 55,000 lanes a mesh, a large mesh
+# among small ones (the mean above it, the others far below), and few small ones among larger ones
+@pytest.mark.parametrize("shapes,precision,by_mesh", [
+    ([(52, 22)] * 2, "fp32", True), ([(52, 20)] * 2, "fp32", False), ([(48, 12)] * 2, "fp64", True), ([(48, 11)] * 2, "fp64", False),
+    ([(48, 128)] + [(5, 2)] * 4, "fp32", False), ([(50, 16)] * 4 + [(5, 2)] * 4, "fp64", False),
+    ([(50, 36)] * 7 + [(5, 2)], "fp32_kahan", True), ([(48, 128)] * 2 + [(5, 2)], "fp32", True)])
+def test_which_batches_go_mesh_by_mesh(shapes, precision, by_mesh):
+    kinds = {s: _mesh(*s) for s in set(shapes)}
+    with eng.Engine([kinds[s] for s in shapes], precision) as e:
+        assert (e.stats()["kernel_family"] == 9) == by_mesh
+        e.step(2)
+        assert e.steps_done == 2
