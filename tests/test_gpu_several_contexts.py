@@ -55,3 +55,58 @@ def test_a_later_context_leaves_an_earlier_one_stepping(precision, shots, first,
     for x, y in zip(want, got):
         assert np.array_equal(x, y)
     assert np.abs(want[5]).max() > 0
+
+
+@pytest.mark.parametrize("kinds", [
+    # each wants every SM for its resident step
+    [("fp64", 1, 150), ("fp64", 1, 150)], [("fp32", 1, 190), ("fp64_ref", 1, 122), ("fp32_kahan", 2, 120)],
+    # beside a wavefront on resident blocks, a batch in one cooperative launch, and two-launch steps
+    [("fp64", 1, 100), ("fp32", 64, 90), ("fp32", 5, 150)], [("fp32", 3, 40), ("batch", 0, 0), ("fp64", 1, 16)]])
+def test_contexts_step_side_by_side_in_threads(kinds, monkeypatch):
+    """Contexts stepped from a thread each, at the same time, give the values they give alone."""
+    import threading
+
+    monkeypatch.setenv("DG_MX_PERSISTENT", "1")  # batches only
+
+    def make(kind):
+        if kind[0] == "batch":
+            return eng.Engine([_long(60, 4, "fp32"), _long(30, 1, "fp32")], "fp32")
+        return eng.Engine(_long(kind[2], kind[1], kind[0]), kind[0])
+
+    def steps(e):
+        for _ in range(40):
+            e.step(7)
+            e.step_async(3)
+        e.synchronize()
+        for f in FIELDS:
+            out.setdefault(id(e), []).append(e.fetch(f, 0, e.info[0]["S"] - 1))
+
+    def work(e):
+        try:
+            steps(e)
+        except Exception as err:  # noqa: BLE001
+            errors.append(err)
+
+    out, errors = {}, []
+    alone, together = [make(k) for k in kinds], [make(k) for k in kinds]
+    for e in alone + together:
+        _load(e)
+    for e in alone:
+        work(e)
+    threads = [threading.Thread(target=work, args=(e,)) for e in together]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for a, b in zip(alone, together):
+        for x, y in zip(out[id(a)], out[id(b)]):
+            assert np.array_equal(x, y)
+    for e in alone + together:
+        e.close()
+
+
+def _long(cells, shots, precision):
+    ref = precision == "fp64_ref"
+    w = pkg.workloads.small_square(n_cells=cells, steps=400, shots=shots)
+    return eng.mesh_from_setup(pkg.host.build_setup(w, full=ref), with_ref_ops=ref)
