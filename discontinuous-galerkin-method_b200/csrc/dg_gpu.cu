@@ -148,7 +148,7 @@ struct dg_gpu_ctx {
   // split meshes (dg_gpu_half_step / dg_gpu_halo_*): the velocity half of a step has run and its
   // stress half has not; per mesh the internal elements sent to and received from other parts
   bool half_pending = false;
-  // one-mesh steps with the wave field resident in shared memory (k_step_resident), many steps a
+  // one-mesh steps with the wave field resident in registers (k_step_resident), many steps a
   // launch: grid, threads, dynamic shared memory, the next launch's first message tag, and the
   // error word (pinned host memory, so that the host reads it without a copy)
   bool resident = false;
@@ -743,8 +743,8 @@ template <class R> void fill_ops(Ops<R>& o, const dg_gpu_mesh& m) {
     }
 }
 
-// Whether the state and the elements' constants of all meshes leave L2 (126 MB) between one sweep and
-// the next.  There the two halves sweep in opposite directions (us a step, 133 MB: 388,000 elements
+// Whether the state and the elements' constants of all meshes are too large to stay in L2 from one
+// sweep to the next: from 75 MB on, the measured crossover (L2 has 126 MB).  There the two halves sweep in opposite directions (us a step, 133 MB: 388,000 elements
 // FP64 69.9 -> 62.9; 81 MB: 80,000 x 8 42.4 -> 40.2; 105 MB: 627,000 FP32 60.5 -> 52.9; 563 MB: 2 M Kahan
 // 279 -> 270; 12 uneven meshes, 620 MB 400 -> 392), and the wavefront step alternates (200,000 x 64
 // 688 -> 675, 102,000 x 16 Kahan 168 -> 160, 49,400 x 24 82 -> 76); it costs
@@ -819,7 +819,7 @@ __global__ void k_wave_sync(const Counters* __restrict__ ctr, unsigned long long
 // Schedule of the wavefront step for the current block size.  A unit is one warp's 32 threads of
 // the element range (thread g works on element g / H, H = shots / 2); the wait list holds, per unit, the
 // distinct units covering one of its elements or a neighbour of one; the lag L (in blocks) covers
-// the unit bandwidth plus a margin of about 60 % of the resident warps, so a stress update
+// the unit bandwidth plus a margin of 12 or 14 warps per SM (16 are resident), so a stress update
 // seldom waits.  Receivers are listed under every unit that covers their element.
 int build_wave(dg_gpu_ctx* c) {
   const MeshHostInfo& h = c->mi[0];
@@ -1055,14 +1055,14 @@ const void* resident_kernel(const dg_gpu_ctx* c, int* max_threads = nullptr) {
   const bool small = c->res_threads <= 256;
   if (c->precision == DG_FP64_REF) return of(kernel_resident_ref());
   if (c->is_double) return of(kernel_resident_d(small));
-  return c->x2 == 1 ? of(kernel_resident_f1(c->kahan, small)) : of(kernel_resident_f2(c->kahan, small));
+  return c->x2 == 1 ? of(kernel_resident_f1(c->kahan)) : of(kernel_resident_f2(c->kahan, small));
 }
 
 // Lanes a block of the resident step can hold, and whether a mesh of K elements of H lanes fits.
 int resident_lanes(const dg_gpu_ctx* c, bool is_double, bool one, bool kahan) {
   if (c->precision == DG_FP64_REF) return kernel_resident_ref().max_threads;
   if (is_double) return kernel_resident_d(false).max_threads;
-  return one ? kernel_resident_f1(kahan, false).max_threads : kernel_resident_f2(kahan, false).max_threads;
+  return one ? kernel_resident_f1(kahan).max_threads : kernel_resident_f2(kahan, false).max_threads;
 }
 constexpr unsigned kResidentSpins = 1u << 20;  // poll limit: a million polls of an L2 line, about a second
 bool resident_off() {
@@ -1282,7 +1282,7 @@ int launch_step(dg_gpu_ctx* c, cudaEvent_t before_t = nullptr, cudaEvent_t mid =
     if (c->multi) DG_TWO(k, c->ops_d, c->md_d[0], c->d_tab_d, c->d_btab_v, c->d_btab_t);
     else DG_TWO(k, c->ops_d, c->md_d[0], (const MeshDev<double>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
   } else if (c->wave && halves != 3) {  // half steps of a wave_mid context
-    const HalfPair<GenFn<float>> k = kernels_fp32_p2(c->kahan, true);
+    const HalfPair<GenFn<float>> k = kernels_fp32_p2(c->kahan);
     DG_TWO(k, c->ops_f, c->md_f[0], (const MeshDev<float>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
   } else if (c->wave) {  // the whole step in one launch: it is timed as the "velocity" interval
     int rc = launch_wave(c);
@@ -1301,7 +1301,7 @@ int launch_step(dg_gpu_ctx* c, cudaEvent_t before_t = nullptr, cudaEvent_t mid =
     int rc = launch_x2(c, mid, hv, ht);
     if (rc) return rc;
   } else {
-    const HalfPair<GenFn<float>> k = c->gen_p2 ? kernels_fp32_p2(c->kahan, true) : kernels_fp32(c->kahan, c->multi);
+    const HalfPair<GenFn<float>> k = c->gen_p2 ? kernels_fp32_p2(c->kahan) : kernels_fp32(c->kahan, c->multi);
     if (c->multi) DG_TWO(k, c->ops_f, c->md_f[0], c->d_tab_f, c->d_btab_v, c->d_btab_t);
     else DG_TWO(k, c->ops_f, c->md_f[0], (const MeshDev<float>*)nullptr, (const int2*)nullptr, (const int2*)nullptr);
   }

@@ -20,11 +20,9 @@ HalfPair<GenFn<float>> kernels_fp32(bool kahan, bool multi) {
   return {k_velocity<ArithOps<float>, false, false>, k_stress<ArithOps<float>, false, false>};
 }
 
-HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan, bool two) {
-  if (two && kahan) return {k_velocity<ArithP2<float2>, true, false>, k_stress<ArithP2<float2>, true, false>};
-  if (two) return {k_velocity<ArithP2<float2>, false, false>, k_stress<ArithP2<float2>, false, false>};
-  if (kahan) return {k_velocity<ArithP2<float>, true, false>, k_stress<ArithP2<float>, true, false>};
-  return {k_velocity<ArithP2<float>, false, false>, k_stress<ArithP2<float>, false, false>};
+HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan) {
+  if (kahan) return {k_velocity<ArithP2<float2>, true, false>, k_stress<ArithP2<float2>, true, false>};
+  return {k_velocity<ArithP2<float2>, false, false>, k_stress<ArithP2<float2>, false, false>};
 }
 
 HalfPair<GenFn<double>> kernels_reference(bool multi, bool otf) {

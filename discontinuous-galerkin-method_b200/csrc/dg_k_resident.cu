@@ -1,12 +1,12 @@
 // dg_k_resident.cu — instances of the resident step (k_step_resident): FP32 one shot and two shots
-// per lane, plain and Kahan, FP64 and the reference
-// operators.  Blocks of up to 256 threads keep all their values in
-// registers; the larger ones serve meshes with more lanes per SM.
+// per lane, plain and Kahan, FP64 and the reference operators.  FP64 and plain FP32 on two shots
+// have a second instance for blocks of up to 256 threads, which keeps all its values in registers
+// (255 and 224 a thread, no spills; 168 and up to 76 bytes of spills at 384 threads).
 #include "dg_kernels.cuh"
 
 namespace dg {
 
-ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan, bool small) {
+ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan) {
   if (kahan) return {k_step_resident<ArithP2<float>, true, 384>, 384};
   return {k_step_resident<ArithP2<float>, false, 512>, 512};
 }

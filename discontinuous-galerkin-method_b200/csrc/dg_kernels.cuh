@@ -38,8 +38,8 @@ template <class F> struct HalfPair {
 
 HalfPair<GenFn<double>> kernels_fp64(bool multi);                 // dg_k_generic.cu
 HalfPair<GenFn<float>> kernels_fp32(bool kahan, bool multi);      // dg_k_generic.cu
-// one FP32 mesh with the compile-time P2 operators, on any layout; `two`: two shots a thread
-HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan, bool two);     // dg_k_generic.cu
+// one FP32 mesh with the compile-time P2 operators, two shots a thread, on any layout
+HalfPair<GenFn<float>> kernels_fp32_p2(bool kahan);               // dg_k_generic.cu
 HalfPair<GenFn<double>> kernels_reference(bool multi, bool otf);  // dg_k_generic.cu
 // S shots (2..128, powers of two), or S = 1 on the one-shot layout
 WaveFn kernel_wave(int S, bool kahan, bool persistent);           // dg_k_wave.cu
@@ -48,9 +48,10 @@ WaveFn kernel_wave(int S, bool kahan, bool persistent);           // dg_k_wave.c
 WaveFn kernel_wave_async(int S, bool kahan);                      // dg_k_wave.cu
 HalfPair<MxFn> kernels_batch(bool kahan);                         // dg_k_multi.cu
 MxpFn kernel_batch_persistent(bool kahan);                        // dg_k_multi.cu
-ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan, bool small);  // dg_k_resident.cu
+// `small`: for blocks of up to 256 threads
+ResKernel<ArithP2<float>> kernel_resident_f1(bool kahan);              // dg_k_resident.cu
 ResKernel<ArithP2<float2>> kernel_resident_f2(bool kahan, bool small); // dg_k_resident.cu
-ResKernel<ArithOps<double>> kernel_resident_d(bool small);            // dg_k_resident.cu
+ResKernel<ArithOps<double>> kernel_resident_d(bool small);             // dg_k_resident.cu
 ResKernel<ArithRef> kernel_resident_ref();                         // dg_k_resident.cu
 
 // the packed instances, split by shot count over three translation units
