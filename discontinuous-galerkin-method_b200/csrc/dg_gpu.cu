@@ -1080,7 +1080,9 @@ int alloc_error_word(dg_gpu_ctx* c) {
 // shot 56,832): elements cut into runs
 // of consecutive ones, one block each; every face between two blocks gets a message slot at the
 // element that receives it (numbered in element order, so a block's messages lie together).  A
-// mesh whose face codes are not mutual, or that does not fit, keeps the two-launch step.
+// mesh whose face codes are not mutual, whose blocks' lanes and messages do not fit into shared memory
+// (many faces between blocks: 7,000 elements of 16 shots in the wavefront step's order), or that does
+// not fit otherwise keeps its other form.
 // Blocks of 128 lanes, one warp per scheduler, as long as there are SMs for them: 64 lanes run
 // 1-5 % slower on 500-3,000 elements (more messages), 256 up to 25 % (warps share schedulers).
 // Against two launches a step, same bits (us a step): 512 elements FP64 11.7 -> 4.3 (20-step calls),
