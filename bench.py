@@ -390,6 +390,8 @@ def run_ours(args):
     e = eng.Engine(meshes, args.precision, device=device, variant=args.variant)
     st = e.stats()
     bytes_step, dof_step = st["bytes_per_step"], st["dof_per_step"]
+    wbytes = 8 if args.precision == "fp64" else 4
+    state_bytes = sum(30 * x.K * x.shots for x in ws) * (wbytes + (4 if args.precision == "fp32_kahan" else 0))
     e.step(W_steps)
     # K steps through the call a user makes (CUDA graphs, or one persistent launch), timed with
     # CUDA events on the context's stream around the whole run
@@ -407,7 +409,9 @@ def run_ours(args):
     launches = e.stats()["launches"]
     value, t_max = job_value(dof_step, K_steps, total_ms, dist, device)
     dof_job = sum_over_ranks(dof_step, dist, device)
-    names = eng.KERNEL_NAMES[st["kernel_family"]]
+    names = (eng.RESIDENT_NAME, None) if st["resident"] else eng.KERNEL_NAMES[st["kernel_family"]]
+    if st["resident"]:  # the wave field goes in and out once a call
+        bytes_step = 2.0 * state_bytes / K_steps
     if names[1] is None:
         # the whole step in one launch (or the whole run in one persistent launch): the kernel's
         # time per step is the timed region's, on the stream it runs on
@@ -431,8 +435,6 @@ def run_ours(args):
     S_tot = sum(x.shots for x in ws)
     K_tot = sum(x.K for x in ws)
     R_tot = sum(x.shots * x.rec.shape[0] for x in ws)
-    wbytes = 8 if args.precision == "fp64" else 4
-    state_bytes = sum(30 * x.K * x.shots for x in ws) * (wbytes + (4 if args.precision == "fp32_kahan" else 0))
 
     # ---- end to end through the public API with pinned host buffers ------------------------
     e.reset()
@@ -566,7 +568,8 @@ def run_ours(args):
             "dtype": {"fp32": "f32", "fp32_kahan": "f32 (Kahan-compensated)", "fp64": "f64"}[args.precision],
             "data": "synthetic (seeded meshes and media)",
             "config": {"workload": desc, "meshes": len(ws), "K": K_tot, "shots": S_tot, "precision": args.precision,
-                       "kernels": eng.KERNEL_FAMILIES[st["kernel_family"]], "variant": args.variant,
+                       "kernels": eng.RESIDENT_FAMILY if st["resident"] else eng.KERNEL_FAMILIES[st["kernel_family"]],
+                       "variant": args.variant,
                        "parallelism": ("single GPU" if world == 1 else
                                        {"weak": "one job of %d shots, 64 contiguous shots per GPU (shard_shots)"
                                                 % (64 * world),
@@ -577,7 +580,7 @@ def run_ours(args):
                        if state_bytes > 126e6 * 1.5 else "state smaller than L2 (not flushed)",
                        "block_threads": st["block_threads"]},
             "gpu_launches": launches,
-            "roofline": {"bound": "hbm", "kernel": dom[0], "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "latency" if st["resident"] else "hbm", "kernel": dom[0], "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
                          "bytes_per_launch": dom[1], "ms_per_launch": dom[2], "time_source": time_source,
                          "step_GBs": bytes_step / (t_max / K_steps * 1e-3) / 1e9,
@@ -589,11 +592,13 @@ def run_ours(args):
                            "GBs": st1["bytes_per_step"] / (tot1 / K_steps * 1e-3) / 1e9,
                            "ratio_batched_over_fp64_plain": value / world / fp64_value,
                            "value_same_timing": fp64_same,
-                           "same_timing": "one dg_gpu_step(%d) call, CUDA graphs, events around the call, no "
+                           "same_timing": "one dg_gpu_step(%d) call, %s, events around the call, no "
                                           "flush: the timing of `value`; FP64 state %.0f MB (L2 126 MB)"
-                                          % (K_steps, fp64_state / 1e6),
+                                          % (K_steps, "resident" if st1["resident"] else "CUDA graphs",
+                                             fp64_state / 1e6),
                            "ms_per_step_same_timing": same1 / K_steps,
-                           "GBs_same_timing": st1["bytes_per_step"] / (same1 / K_steps * 1e-3) / 1e9,
+                           "GBs_same_timing": None if st1["resident"] else
+                           st1["bytes_per_step"] / (same1 / K_steps * 1e-3) / 1e9,
                            "ratio_same_timing": value / world / fp64_same},
             "accuracy": accuracy,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

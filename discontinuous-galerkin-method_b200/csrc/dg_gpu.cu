@@ -2736,6 +2736,7 @@ int dg_gpu_stats_get(dg_gpu_ctx* c, dg_gpu_stats* out) {
                      : (c->mx ? (c->mx_persistent ? 8 : 4)
                               : (c->gen_p2 ? 1 : (c->x2 == 1 ? 3 : (c->x2 ? (c->x2pm ? 7 : 2) : 1)))));
   if (!c->subs.empty()) c->stats.kernel_family = 9;
+  c->stats.resident = c->resident;
   c->stats.bytes_per_step = c->wave ? c->bytes_wave : c->bytes_two_pass;
   *out = c->stats;
   return DG_OK;

@@ -84,7 +84,8 @@ class _Opts(C.Structure):
 class _Stats(C.Structure):
     _fields_ = [("ms_velocity", C.c_double), ("ms_stress", C.c_double), ("launches", C.c_long),
                 ("steps_done", C.c_long), ("block_threads", C.c_int), ("graph_steps", C.c_int),
-                ("bytes_per_step", C.c_double), ("dof_per_step", C.c_double), ("kernel_family", C.c_int)]
+                ("bytes_per_step", C.c_double), ("dof_per_step", C.c_double), ("kernel_family", C.c_int),
+                ("resident", C.c_int)]
 
 KERNEL_FAMILIES = {0: "reference operators (k_velocity_ref/k_stress_ref)",
                    1: "one (element, shot) per thread (k_velocity/k_stress)",
@@ -104,6 +105,8 @@ KERNEL_NAMES = {0: ("k_velocity_ref", "k_stress_ref"), 1: ("k_velocity", "k_stre
                 4: ("k_velocity_mx", "k_stress_mx"), 5: ("k_step_wave", None),
                 6: ("k_step_wave_p", None), 7: ("k_velocity_x2", "k_stress_x2"), 8: ("k_step_mx_p", None),
                 9: ("k_velocity/k_stress of each mesh", None)}
+# the step calls of a context whose stats say `resident`
+RESIDENT_NAME, RESIDENT_FAMILY = "k_step_resident", "one mesh held on the SMs for a whole step call (k_step_resident)"
 
 
 _LIB = None

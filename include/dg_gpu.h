@@ -131,9 +131,11 @@ typedef struct {
 	                            lanes a mesh on average, 50,000 with no mesh counted for more than
 	                            90,000, a lane being one element and shot in FP64, one element and two
 	                            shots in FP32).
-	                          A single mesh whose state fits in the SMs' registers runs dg_gpu_step in one
-	                          cooperative launch for all its steps; the family reported is then that of
-	                          its other calls (half steps, timed and profiled steps), with the same bits */
+	                          Of a resident context (below): the family of its other calls */
+	int resident;          /* 1: a single mesh whose state fits in the SMs' registers: dg_gpu_step, _step_async
+	                          and _step_snapshots run their steps in one cooperative launch a call
+	                          (k_step_resident; graph_steps and bytes_per_step say nothing of it).  Half
+	                          steps, timed, profiled and captured steps run kernel_family, the same bits */
 } dg_gpu_stats;
 
 void dg_gpu_default_opts(dg_gpu_opts *opts);

@@ -52,3 +52,15 @@ def test_binding_constants_equal_header():
         assert defs[name] == value, name
     for code, name in e.ERRORS.items():
         assert defs[name] == code, name
+
+
+def test_stats_layout_equals_header():
+    """The binding's dg_gpu_stats has the header's fields, in its order and of its size."""
+    with open(os.path.join(ROOT, "include", "dg_gpu.h")) as f:
+        text = re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S)
+    body = text[:text.index("} dg_gpu_stats;")]
+    body = body[body.rindex("{") + 1:]
+    ctype = {"double": ctypes.c_double, "long": ctypes.c_long, "int": ctypes.c_int}
+    want = [(n.strip(), ctype[t]) for t, names in re.findall(r"\b(double|long|int)\s+([^;]+);", body) for n in names.split(",")]
+    assert [tuple(f) for f in pkg.engine._Stats._fields_] == want
+    assert ctypes.sizeof(pkg.engine._Stats) == 64  # what callers of the first release allocate

@@ -43,11 +43,11 @@ def test_the_resident_step_up_to_its_last_lane(precision, cells, shots, monkeypa
     stats, got = _run(m, precision)
     lanes = shots if precision.startswith("fp64") or shots == 1 else (shots + 1) // 2
     per_sm = -(-2 * cells * cells // 148) * lanes  # the most a block holds
-    assert (stats["launches"] == 1) == (per_sm <= LANES[precision, shots == 1])
+    assert (stats["launches"] == 1) == bool(stats["resident"]) == (per_sm <= LANES[precision, shots == 1])
     assert stats["launches"] in (1, 2 * STEPS)
     monkeypatch.setenv("DG_RESIDENT", "0")
     stats, want = _run(m, precision)
-    assert stats["launches"] == 2 * STEPS
+    assert not stats["resident"] and stats["launches"] == 2 * STEPS
     for a, b in zip(want, got):
         assert np.array_equal(a, b)
 
