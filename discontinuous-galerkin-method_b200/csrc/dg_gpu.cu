@@ -219,6 +219,7 @@ struct dg_gpu_ctx {
   // event after its last copy, waited for before the half is used again
   static constexpr int kWave = 256;  // doubles a half
   double* wave_host = nullptr;
+  unsigned char* pinned = nullptr;  // two pages of pinned memory: the resident step's error word, that staging
   int wave_half = 0, wave_pos = 0;  // where the next update goes
   long staged_end = 0;              // end of the samples whose copies may still be on their way
   cudaEvent_t ev_wave[2] = {nullptr, nullptr};
@@ -237,10 +238,13 @@ struct dg_gpu_ctx {
     if (ev_fetch) cudaEventDestroy(ev_fetch);
     if (ev_wavelet) cudaEventDestroy(ev_wavelet);
     if (snap_host) cudaFreeHost(snap_host);
-    if (res_error) cudaFreeHost(res_error);
     for (auto& e : ev_wave)
       if (e) cudaEventDestroy(e);
-    if (wave_host) cudaFreeHost(wave_host);
+    if (pinned) {
+      cudaStreamSynchronize(stream);
+      cudaHostUnregister(pinned);
+      free(pinned);
+    }
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     for (void* p : allocs) cudaFree(p);
@@ -258,6 +262,23 @@ struct dg_gpu_ctx {
     int rc = alloc(out, h.size());
     if (rc) return rc;
     if (!h.empty()) CK(cudaMemcpyAsync(*out, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
+    return DG_OK;
+  }
+  // The two pinned pages.  Registered, not allocated pinned: 0.4 ms against 1 to 3 (20 contexts, as they are
+  // made one after the other).
+  int ensure_pinned() {
+    if (pinned) return DG_OK;
+    constexpr size_t page = 4096;
+    static_assert(2 * kWave * sizeof(double) <= page, "the staging fits a page");
+    void* p = aligned_alloc(page, 2 * page);
+    if (!p) return fail(DG_ERR_NOMEM, "pinned pages");
+    memset(p, 0, 2 * page);
+    const cudaError_t e = cudaHostRegister(p, 2 * page, cudaHostRegisterMapped);
+    if (e != cudaSuccess) {
+      free(p);
+      return cuda_fail(e, "cudaHostRegister", __LINE__);
+    }
+    pinned = (unsigned char*)p;
     return DG_OK;
   }
   // free one buffer made by alloc/upload (after the stream has finished with it)
@@ -1070,11 +1091,6 @@ bool resident_off() {
   return env && atoi(env) == 0;
 }
 
-int alloc_error_word(dg_gpu_ctx* c) {
-  CK(cudaHostAlloc(&c->res_error, sizeof(int), cudaHostAllocMapped));
-  return DG_OK;
-}
-
 // The resident step's tables, where a thread for every lane fits on the SMs at once (FP64 and two
 // shots a lane: 56,832 lanes, FP32 one shot 75,776, Kahan and the reference operators 37,888, Kahan one
 // shot 56,832): elements cut into runs
@@ -1193,16 +1209,16 @@ int build_resident(dg_gpu_ctx* c) {
   if ((rc = c->upload(&d_start, start)) || (rc = c->upload(&d_slots, sstart)) || (rc = c->upload(&d_link, link)) ||
       (rc = c->upload(&d_out, out)) || (rc = c->upload(&d_rs, rstart)) || (rc = c->upload(&d_rl, rlist)) ||
       (rc = c->alloc(&w.pt, mt * w.ps)) || (rc = c->alloc(&w.pv, mv * w.ps)) || (rc = c->alloc(&w.arrived, 1)) ||
-      (rc = alloc_error_word(c))) {
+      (rc = c->ensure_pinned())) {
     while (c->allocs.size() > held) c->release(c->allocs.back());
     c->rs = Resident{};
     c->res_stalled = -1;
-    return rc == DG_ERR_NOMEM ? DG_OK : rc;
+    return rc == DG_ERR_NOMEM || !c->pinned ? DG_OK : rc;
   }
   CK(cudaMemsetAsync(w.pt, 0, mt * w.ps * sizeof(uint4), c->stream));
   CK(cudaMemsetAsync(w.pv, 0, mv * w.ps * sizeof(uint4), c->stream));
   CK(cudaMemsetAsync(w.arrived, 0, sizeof(unsigned), c->stream));
-  *c->res_error = 0;
+  c->res_error = (int*)c->pinned;
   CK(cudaHostGetDevicePointer(&w.error, c->res_error, 0));
   w.e_start = d_start;
   w.s_start = d_slots;
@@ -2647,6 +2663,16 @@ int dg_gpu_debug_stall_wave(dg_gpu_ctx* c, int unit) {
   return DG_OK;
 }
 
+// The staging of small updates; without it they go the way of the longer ones.
+static int ensure_wavelet_staging(dg_gpu_ctx* c) {
+  if (c->wave_host) return DG_OK;
+  int rc = c->ensure_pinned();
+  for (auto& e : c->ev_wave)
+    if (!rc) rc = ensure_event(&e);
+  if (!rc) c->wave_host = (double*)(c->pinned + 4096);
+  return rc;
+}
+
 int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w) {
   if (!c || !w || mesh < DG_ALL_MESHES || mesh >= (int)c->mi.size() || t0 < 0 || n < 0)
     return fail(DG_ERR_ARG, "bad arguments");
@@ -2670,13 +2696,7 @@ int dg_gpu_set_wavelet(dg_gpu_ctx* c, int mesh, long t0, long n, const double* w
   // stream, behind the steps enqueued and ahead of the next, without a wait (1.8 us a call against
   // 8 with the copy stream, its event and the wait)
   const long few = (long)(k1 - k0) * n;
-  if (few > 0 && few <= 64) {
-    if (!c->wave_host) {
-      void* p = nullptr;
-      CK(cudaMallocHost(&p, 2 * dg_gpu_ctx::kWave * sizeof(double)));
-      c->wave_host = (double*)p;
-      for (auto& e : c->ev_wave) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
+  if (few > 0 && few <= 64 && ensure_wavelet_staging(c) == DG_OK) {
     if (c->wave_pos + few > dg_gpu_ctx::kWave) {  // the half is full: on to the other
       CK(cudaEventRecord(c->ev_wave[c->wave_half], c->stream));
       c->wave_half ^= 1;
