@@ -152,8 +152,8 @@ int dg_gpu_step(dg_gpu_ctx *ctx, long n);
  * watchdog on, its checks still wait): the host is free until dg_gpu_synchronize, which waits
  * and reports a wait limit reached on the way (DG_ERR_TIMEOUT).  Every other call of the context
  * is ordered after the enqueued steps (fetches wait for them), except dg_gpu_fetch_traces of
- * steps an earlier step call completes and dg_gpu_set_wavelet of samples no enqueued step reads,
- * which run on a second stream while the later steps keep running.
+ * steps an earlier step call completes and dg_gpu_set_wavelet of more than 64 samples that no
+ * enqueued step reads, which run on a second stream while the later steps keep running.
  * A caller that captures the context's stream (dg_gpu_context_stream) gets the steps as launches
  * that take the step number from the device, so the capture can be replayed: each replay advances
  * the wave field by the captured steps, and calls made later go on from there.  The host counts a
