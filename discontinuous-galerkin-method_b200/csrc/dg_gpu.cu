@@ -1997,10 +1997,11 @@ static int enqueue_subs(dg_gpu_ctx* c, long n) {
   // in a call of many steps no more chains than keep their states in L2 together (4 meshes of
   // 28,800 elements, 8 shots, 28 MB each: two chains 43.1 us a step, four 62.2); in a short one
   // the gaps between launches cost more (24 meshes of 20,000, 8 shots, 5 steps a call: 265, 231).
-  // There a mesh below kBatchLanes takes about 15 us of its chain whatever its size, so those have
-  // chains of their own (calls of one: 6 uneven meshes of 3,000 to 188,000 lanes FP32 106 -> 80, FP64
-  // 169 -> 142; all meshes in one launch 91 and 148; twelve chains for all meshes cost 24 of 80,000
-  // lanes 297 instead of 268)
+  // In calls of a few a mesh below kBatchLanes takes about 15 us of its chain whatever its size, so those
+  // have chains of their own (calls of one: 6 uneven meshes of 3,000 to 188,000 lanes FP32 107 -> 86,
+  // FP64 169 -> 144; all meshes in one launch 91 and 148; of four: 92 -> 71, 152 -> 134; from six on the
+  // graphs close the gaps and more chains cost the larger batches 1 to 3 %: 12 meshes FP32 363 -> 374;
+  // twelve chains for all meshes cost 24 of 80,000 lanes 297 instead of 268 in calls of one)
   int chains = kChains;
   if (n >= 16) {
     double held = 0;
@@ -2020,7 +2021,7 @@ static int enqueue_subs(dg_gpu_ctx* c, long n) {
     const long m = std::min(n, sub->max_steps - sub->t);
     if (m <= 0) continue;  // past its last step
     const double lanes = batch_lanes(c->precision, sub->mi[0].K, sub->mi[0].S_pad);
-    const bool alone = bytes(k) > kAlone, own = n < 16 && lanes < kBatchLanes;
+    const bool alone = bytes(k) > kAlone, own = n < 6 && lanes < kBatchLanes;
     const int first = own ? kChains : 0, past = own ? kAll : chains;
     const int at = (int)(std::min_element(load + first, load + past) - load);
     CK(cudaStreamWaitEvent(sub->stream, last[at], 0));

@@ -20,7 +20,7 @@ def _mesh(cells, shots):
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 def test_calls_of_any_length(precision, monkeypatch):
     """Two meshes of more than 50,000 lanes and eighteen small ones (more than there are chains for
-    those), in calls of 1, 15, 16 and 8 steps, against launches over all meshes."""
+    those), in calls of 1, 5, 15, 16 and 3 steps, against launches over all meshes."""
     large = (115, 4) if precision == "fp32" else (115, 2)
     meshes = [_mesh(*s) for s in [(4 + k, 1 + k % 3) for k in range(9)] + [large, (115, 5)] + [(5 + k, 2) for k in range(9)]]
     out = []
@@ -32,7 +32,7 @@ def test_calls_of_any_length(precision, monkeypatch):
             for k, info in enumerate(e.info):
                 for f in FIELDS:
                     e.load(f, rng.standard_normal(info["K"] * 6) * (1e-3 if f[0] == "V" else 1e3), k, info["S"] - 1)
-            for n in (1, 15, 16, 8):
+            for n in (1, 5, 15, 16, 3):
                 e.step(n)
             out.append([e.fetch(f, k, eng.ALL_SHOTS) for k in range(len(meshes)) for f in FIELDS] +
                        list(e.fetch_traces(0, STEPS, eng.ALL_MESHES)))
