@@ -219,7 +219,7 @@ struct dg_gpu_ctx {
   // event after its last copy, waited for before the half is used again
   static constexpr int kWave = 256;  // doubles a half
   double* wave_host = nullptr;
-  unsigned char* pinned = nullptr;  // two pages of pinned memory: the resident step's error word, that staging
+  unsigned char* pinned = nullptr;  // mapped pinned memory: the resident step's error word, at 64 that staging
   int wave_half = 0, wave_pos = 0;  // where the next update goes
   long staged_end = 0;              // end of the samples whose copies may still be on their way
   cudaEvent_t ev_wave[2] = {nullptr, nullptr};
@@ -240,11 +240,7 @@ struct dg_gpu_ctx {
     if (snap_host) cudaFreeHost(snap_host);
     for (auto& e : ev_wave)
       if (e) cudaEventDestroy(e);
-    if (pinned) {
-      cudaStreamSynchronize(stream);
-      cudaHostUnregister(pinned);
-      free(pinned);
-    }
+    if (pinned) cudaFreeHost(pinned);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     for (void* p : allocs) cudaFree(p);
@@ -264,20 +260,14 @@ struct dg_gpu_ctx {
     if (!h.empty()) CK(cudaMemcpyAsync(*out, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
     return DG_OK;
   }
-  // The two pinned pages.  Registered, not allocated pinned: 0.4 ms against 1 to 3 (20 contexts, as they are
-  // made one after the other).
+  // The pinned block.  Allocated: 0.05 ms where the process holds pinned memory already (CUDA takes it
+  // from a larger piece), 1 to 3 ms where it does not; registering two pages takes 0.4 ms and more
+  // either way (512 elements, making a context beside other pinned buffers: 0.5 against 0.9 to 3.5 ms).
   int ensure_pinned() {
     if (pinned) return DG_OK;
-    constexpr size_t page = 4096;
-    static_assert(2 * kWave * sizeof(double) <= page, "the staging fits a page");
-    void* p = aligned_alloc(page, 2 * page);
-    if (!p) return fail(DG_ERR_NOMEM, "pinned pages");
-    memset(p, 0, 2 * page);
-    const cudaError_t e = cudaHostRegister(p, 2 * page, cudaHostRegisterMapped);
-    if (e != cudaSuccess) {
-      free(p);
-      return cuda_fail(e, "cudaHostRegister", __LINE__);
-    }
+    void* p = nullptr;
+    CK(cudaHostAlloc(&p, 64 + 2 * kWave * sizeof(double), cudaHostAllocMapped));
+    memset(p, 0, 64);
     pinned = (unsigned char*)p;
     return DG_OK;
   }
@@ -2670,7 +2660,7 @@ static int ensure_wavelet_staging(dg_gpu_ctx* c) {
   int rc = c->ensure_pinned();
   for (auto& e : c->ev_wave)
     if (!rc) rc = ensure_event(&e);
-  if (!rc) c->wave_host = (double*)(c->pinned + 4096);
+  if (!rc) c->wave_host = (double*)(c->pinned + 64);
   return rc;
 }
 
