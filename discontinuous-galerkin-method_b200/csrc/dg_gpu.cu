@@ -1057,12 +1057,9 @@ int launch_wave(dg_gpu_ctx* c) {
   return DG_OK;
 }
 
-// the resident step's kernel for this context's arithmetic, and the threads its registers allow
-const void* resident_kernel(const dg_gpu_ctx* c, int* max_threads = nullptr) {
-  auto of = [&](auto k) {
-    if (max_threads) *max_threads = k.max_threads;
-    return (const void*)k.fn;
-  };
+// the resident step's kernel for this context's arithmetic; `count`: the step from the device's counter
+const void* resident_kernel(const dg_gpu_ctx* c, bool count) {
+  auto of = [&](auto k) { return (const void*)k.fn[count]; };
   const bool small = c->res_threads <= 256;
   if (c->precision == DG_FP64_REF) return of(kernel_resident_ref());
   if (c->is_double) return of(kernel_resident_d(small));
@@ -1172,13 +1169,15 @@ int build_resident(dg_gpu_ctx* c) {
   if (c->res_smem > (size_t)smem_max || 6L * w.nls > 65535) return DG_OK;
   c->res_blocks = nb;
   c->res_threads = (int)std::min<long>(max_threads, (w.nl + 31) / 32 * 32 + (most * H + 31) / 32 * 32);
-  const void* kernel = resident_kernel(c);
-  // the limit belongs to the kernel, which other contexts of this process launch with other sizes:
-  // always the device's
-  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, c->res_threads, c->res_smem));
-  if ((long)per_sm * c->num_sms < nb) return DG_OK;
+  for (bool count : {false, true}) {
+    const void* kernel = resident_kernel(c, count);
+    // the limit belongs to the kernel, which other contexts of this process launch with other sizes:
+    // always the device's
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, c->res_threads, c->res_smem));
+    if ((long)per_sm * c->num_sms < nb) return DG_OK;
+  }
   // test hook: one face's messages go to a slot nobody reads, and waits give up early
   if (getenv("DG_RESIDENT_STALL") && slots > 0) {
     for (long e = 0; e < K && w.spin_limit > 4096; e++)
@@ -1233,13 +1232,13 @@ int resident_unstall(dg_gpu_ctx* c) {
 
 // nsteps steps in one launch (cooperative: blocks wait for one another's messages)
 int launch_resident(dg_gpu_ctx* c, int nsteps) {
-  long long from = c->may_replay ? -1 : c->t;
+  long long t0 = c->t;
   unsigned seq = c->res_seq;
   void* ops = c->is_double ? (void*)&c->ops_d : (void*)&c->ops_f;  // FP32: operators are constants
   void* mesh = c->is_double ? (void*)&c->md_d[0] : (void*)&c->md_f[0];
-  void* args[] = {ops, mesh, &c->rs, &c->d_ctr, &from, &nsteps, &seq};
+  void* args[] = {ops, mesh, &c->rs, &c->d_ctr, &t0, &nsteps, &seq};
   c->res_seq += (unsigned)nsteps + 1u;
-  CK(cudaLaunchCooperativeKernel(resident_kernel(c), dim3(c->res_blocks), dim3(c->res_threads), args, c->res_smem,
+  CK(cudaLaunchCooperativeKernel(resident_kernel(c, c->may_replay), dim3(c->res_blocks), dim3(c->res_threads), args, c->res_smem,
                                  c->stream));
   return DG_OK;
 }

@@ -27,7 +27,7 @@ using MxpFn = void (*)(Ops<float>, Ops2, const MeshDev<float>*, MxLoop, Counters
 template <class A>
 using ResFn = void (*)(typename A::Ops, MeshDev<typename A::R>, Resident, Counters*, long long, int, unsigned);
 template <class A> struct ResKernel {
-  ResFn<A> fn;
+  ResFn<A> fn[2];   // the step number from the host, and from the device's counter
   int max_threads;  // threads per block its registers allow
 };
 

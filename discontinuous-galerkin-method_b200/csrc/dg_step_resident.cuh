@@ -158,24 +158,23 @@ struct ArithRef {
 template <class A> constexpr bool is_ref = false;
 template <> constexpr bool is_ref<ArithRef> = true;
 
-// `nsteps` steps from step `from`, or, if that is negative (the device's counter may be ahead of the host:
-// a caller replays captured steps), from the step the counter holds, as the other forms of the step
-// take it.  The counter costs a one-step call 0.5 us (its load, and the blocks counting themselves so
-// that the last to have read it advances it), so it is read only there.  The stresses held between two steps carry the sponge factor of
+// `nsteps` steps from step t0, or, COUNT (the device's counter may be ahead of the host: a caller replays
+// captured steps), from the step the counter holds, as the other forms of the step take it.  There the
+// blocks count themselves, and the last to have read the counter advances it.  An instance of its own:
+// reading the counter costs a one-step call of 17 us 0.5 us, a run-time choice 0.3.  The stresses held between two steps carry the sponge factor of
 // the coming step already (those in global memory do not), so neighbours read them as they are;
 // the stress tag of step s is seq + s, the velocity tag seq + s + 1.
-template <class A, bool KAHAN, int MAXT>
+template <class A, bool KAHAN, int MAXT, bool COUNT>
 __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant__ typename A::Ops ops,
                                                            const __grid_constant__ MeshDev<typename A::R> m,
                                                            const __grid_constant__ Resident w,
-                                                           Counters* __restrict__ ctr, long long from, int nsteps,
+                                                           Counters* __restrict__ ctr, long long t0, int nsteps,
                                                            unsigned seq) {
   using V = typename A::V;
   using R = typename A::R;
   constexpr int SV = sizeof(V) / sizeof(R);  // shots of a lane
   constexpr bool REF = is_ref<A>;
-  long long t0 = from;
-  if (from < 0) {
+  if constexpr (COUNT) {
     t0 = *(volatile const long long*)&ctr->v;
     nsteps = (int)min((long long)nsteps, m.steps - t0);
     if (nsteps <= 0) return;
@@ -257,10 +256,12 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
           for (int f = 0; f < 3; f++) g[(f * NP + k) * nls] = v[3 * k + f];
       }
       __syncthreads();
-      if (from < 0 && s == 0 && l == 0 && atomicAdd(w.arrived, 1u) == gridDim.x - 1) {
-        *w.arrived = 0;
-        ctr->v = t0 + nsteps;
-        ctr->s = t0 + nsteps - 1;
+      if constexpr (COUNT) {
+        if (s == 0 && l == 0 && atomicAdd(w.arrived, 1u) == gridDim.x - 1) {
+          *w.arrived = 0;
+          ctr->v = t0 + nsteps;
+          ctr->s = t0 + nsteps - 1;
+        }
       }
       if (mine) {
         if constexpr (!REF) {
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_step_resident(const __grid_constant
       for (int p = 0; p < 30; p++) *state_at<V>(m.C, m, e, p, q) = cc[p];
     }
   }
-  if (from >= 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+  if (!COUNT && blockIdx.x == 0 && threadIdx.x == 0) {
     ctr->v = t0 + nsteps;
     ctr->s = t0 + nsteps - 1;
   }
